@@ -128,8 +128,11 @@ struct pe_engine {
     // graph cache
     cudaGraphExec_t gexec = nullptr;
     GraphKey gkey;
+    int graph_launches = 0;
     // occupancy cache
     int bps_cache[2][4][2][9] = {};
+    int lanes_grid = 0;  // grid of the 32-lane shape
+    int wide_bps = 0;    // blocks per SM of the block-per-flight kernel, once both default kernels are set up
     // gradient
     DevBuf<float> g_setup, g_ck, g_adj, g_ybar, g_dist, g_fsum;
     DevBuf<int> g_steps, g_kind, g_order, g_work;
@@ -240,22 +243,62 @@ FlightArgs flight_args(pe_engine* e, int pop, int nseeds, int vary, int max_step
     return a;
 }
 
+int default_kernels(pe_engine* e) {  // occupancy queries and shared-memory opt-ins, outside any capture
+    if (e->wide_bps) return PE_OK;
+    pe_config c = e->cfg;
+    c.blocks = 0; c.formulation = 1; c.reg_cap = 0; c.lanes = 32; c.warps = 4;
+    e->lanes_grid = blocks_for(e, c);
+    PE_CUDA(flight_quad_configure());
+    PE_CUDA(flight_wide_configure(&e->wide_bps));
+    return PE_OK;
+}
+
+// The body-frame flights in the engine's own choice of kernel.
+int enqueue_fly_default(pe_engine* e, int pop, int nseeds, int vary, int max_steps, float* dist, int* steps,
+                        cudaStream_t s, int* launches) {
+    if (int rc = default_kernels(e)) return rc;
+    FlightArgs a = flight_args(e, pop, nseeds, vary, max_steps, dist, steps);
+    a.step_end = max_steps;
+    int* c = e->counters.p;  // queue, flights ended, flights handed over, the second kernel's queue
+    PE_CUDA(cudaMemsetAsync(c, 0, sizeof(int) * 4, s));
+    a.work = c;
+    const long long per_sm = ((long long)a.n_flights + e->nsm - 1) / e->nsm;
+    if (per_sm <= kWideFlights) {
+        PE_CUDA(launch_flight_wide(a, e->nsm, e->wide_bps, s));
+        (*launches)++;
+        return PE_OK;
+    }
+    a.landed = c + 1;
+    a.hand_over = kHandOver * e->nsm;
+    a.active_out = e->list0.p;
+    a.n_active_out = c + 2;
+    if (per_sm <= kLanesFlights)
+        PE_CUDA(launch_flight_fast(a, FlightShape{32, 4, kMaxSteps, 0, 1, 0}, e->lanes_grid, s));
+    else
+        PE_CUDA(launch_flight_quad(a, e->nsm, s));
+    a.landed = nullptr;
+    a.active_in = a.active_out;
+    a.n_active_in = a.n_active_out;
+    a.active_out = nullptr;
+    a.n_active_out = nullptr;
+    a.work = c + 3;
+    PE_CUDA(launch_flight_wide(a, e->nsm, e->wide_bps, s));
+    *launches += 2;
+    return PE_OK;
+}
+
+// Whether a configuration leaves the kernel to the engine: the default shape in one launch.
+bool default_shape(const pe_config& c, int max_steps) {
+    return c.formulation == 1 && c.lanes == 16 && (c.reg_cap == 0 || c.reg_cap == 3) && c.blocks == 0 && max_steps <= c.chunk;
+}
+
 // Enqueue the flights of pop x nseeds (plane table already prepared on this stream).
 int enqueue_fly(pe_engine* e, int pop, int nseeds, int vary, int max_steps, float* dist, int* steps,
                 cudaStream_t s, int* launches) {
     pe_config c = e->cfg;
-    // A batch of at most 192 flights per SM (a holdout of 8 x 128, 1,024 x 8 genomes) flies 32
-    // lanes per flight in 4-warp blocks: with few waves of flights the run is bound by its longest
-    // flights, whose steps finish sooner at 32 lanes (measured on GB300: 15-23 % faster below 160
-    // flights per SM, even near 215, 16 lanes ahead from 320).  The body-frame kernel's results do
-    // not depend on the shape.
-    if (c.formulation == 1 && c.lanes == 16 && (c.reg_cap == 0 || c.reg_cap == 3) && c.blocks == 0 &&
-        (long long)pop * nseeds <= 192LL * e->nsm) {
-        c.lanes = 32;
-        c.warps = 4;
-        c.reg_cap = 0;
-    }
     const int nchunks = (max_steps + c.chunk - 1) / c.chunk;
+    if (default_shape(c, max_steps))
+        return enqueue_fly_default(e, pop, nseeds, vary, max_steps, dist, steps, s, launches);
     int* work = e->counters.p;
     int* nact = e->counters.p + nchunks;
     PE_CUDA(cudaMemsetAsync(e->counters.p, 0, sizeof(int) * (2 * nchunks + 1), s));
@@ -411,7 +454,8 @@ int pe_eval_batch(pe_engine* e, const float* d_genomes, int pop, const int* h_se
         k.genomes = d_genomes; k.dist = dist; k.steps = steps; k.scores = d_scores; k.stream = s;
         k.pop = pop; k.nseeds = nseeds; k.vary = vary; k.max_steps = max_steps; k.smooth = e->smooth; k.cfg = e->cfg;
         if (!e->gexec || !(k == e->gkey)) {
-            blocks_for(e, e->cfg);  // occupancy query outside the capture
+            blocks_for(e, e->cfg);  // occupancy queries outside the capture
+            if (int rc = default_kernels(e)) return rc;
             if (e->gexec) { cudaGraphExecDestroy(e->gexec); e->gexec = nullptr; }
             cudaStream_t cs = s;
             bool own = false;
@@ -431,9 +475,10 @@ int pe_eval_batch(pe_engine* e, const float* d_genomes, int pop, const int* h_se
             cudaGraphDestroy(g);
             if (ce != cudaSuccess) { e->gexec = nullptr; return fail(PE_ECUDA, "graph instantiate: %s", cudaGetErrorString(ce)); }
             e->gkey = k;
+            e->graph_launches = cl;
         }
         PE_CUDA(cudaGraphLaunch(e->gexec, s));
-        launches = 3 + (max_steps + e->cfg.chunk - 1) / e->cfg.chunk + (d_scores ? 1 : 0);
+        launches = e->graph_launches;
     } else {
         if (int rc = enqueue_eval(e, d_genomes, pop, nseeds, vary, max_steps, dist, steps, d_scores, s, &launches))
             return rc;
@@ -505,7 +550,10 @@ int pe_grad(pe_engine* e, const float* d_genomes, int pop, const int* h_seeds, i
     cudaStream_t s = (cudaStream_t)stream;
     const int nf = pop * nseeds;
     const int nck = max_steps / K + 1;
-    if (int rc = engine_reserve(e, pop, 0)) return rc;
+    // the forward pass of a batch that fits its hand-over needs the flight lists and states
+    const bool hand_over = nf <= kGradLanesFlights * e->nsm;
+    if (int rc = engine_reserve(e, pop, hand_over ? nf : 0)) return rc;
+    if (int rc = default_kernels(e)) return rc;
     if (e->g_K != K) {
         PE_CUDA(grad_configure(K, e->g_rev_grid, e->nsm));
         if (!e->g_fwd_bps[0]) PE_CUDA(grad_forward_configure(e->g_fwd_bps));
@@ -518,7 +566,7 @@ int pe_grad(pe_engine* e, const float* d_genomes, int pop, const int* h_seeds, i
     PE_CUDA(e->g_steps.ensure((size_t)nf));
     PE_CUDA(e->g_kind.ensure((size_t)nf));
     PE_CUDA(e->g_order.ensure((size_t)nf));
-    PE_CUDA(e->g_work.ensure(2));
+    PE_CUDA(e->g_work.ensure(kGradCounters));
     if (!d_dist) PE_CUDA(e->g_dist.ensure((size_t)nf));
     // Every step's body force and torque from the forward pass (32 B per flight-step), so the
     // reverse pass recomputes states through the integrator alone, when they fit in 4 GiB;
@@ -573,6 +621,12 @@ int pe_grad(pe_engine* e, const float* d_genomes, int pop, const int* h_seeds, i
     fa.grad_kind = a.kind;
     fa.grad_K = K;
     fa.grad_nck = nck;
+    if (hand_over) {
+        fa.landed = a.work + 2;
+        fa.hand_over = kHandOver * e->nsm;
+        fa.active_out = e->list0.p;
+        fa.n_active_out = a.work + 3;
+    }
     // The reverse pass is bound by its longest flights' chains and by how many flights it keeps in
     // flight.  With the stored forces the flights other than the longest take grad_group_size(K) per
     // block, warp 0 carrying all their integrator chains at once: the longest take the pipelined
@@ -590,10 +644,11 @@ int pe_grad(pe_engine* e, const float* d_genomes, int pop, const int* h_seeds, i
     if (store_forces && grad_long_pass(K) && (small || a.group > 1))
         a.n_long = std::min(nf, std::max(1, a.group > 1 && small ? e->nsm / 4 : e->nsm / 8));
     a.n_single = a.group > 1 ? (group_req == 1 ? nf : e->nsm) : 0;
-    PE_CUDA(launch_grad(a, fa, e->nsm, e->g_fwd_bps, e->g_rev_grid, s, e->ev[2]));
+    PE_CUDA(launch_grad(a, fa, e->nsm, e->g_fwd_bps, e->wide_bps, e->g_rev_grid, s, e->ev[2]));
     PE_CUDA(record_event(e->ev[3], s));
-    // prepare (3), set-up, forward, order, reverse (two kernels with the pipelined pass), weights, genome
-    e->last_launches = 3 + 6 + (a.n_long > 0 ? 1 : 0);
+    // prepare (3), set-up, forward (two kernels with the hand-over), order, reverse (two with the
+    // pipelined pass), weights, genome
+    e->last_launches = 3 + 6 + (hand_over && nf > kWideFlights * e->nsm ? 1 : 0) + (a.n_long > 0 ? 1 : 0);
     e->prepared_pop = pop;
     e->timed = true;
     return PE_OK;

@@ -1531,14 +1531,14 @@ cudaError_t grad_configure(int K, int rev_grid[2], int nsm) {
     return cudaSuccess;
 }
 
-cudaError_t launch_grad(const GradArgs& a, const FlightArgs& fwd, int nsm, const int fwd_bps[2], const int rev_grid[2],
-                        cudaStream_t s, cudaEvent_t mid) {
+cudaError_t launch_grad(const GradArgs& a, const FlightArgs& fwd, int nsm, const int fwd_bps[2], int wide_bps,
+                        const int rev_grid[2], cudaStream_t s, cudaEvent_t mid) {
     const bool grouped = a.group > 1;
     if (grouped && (a.group != kRevGroup || !a.fsum || rev_grid[1] <= 0)) return cudaErrorInvalidValue;
-    cudaError_t e = cudaMemsetAsync(a.work, 0, 2 * sizeof(int), s);
+    cudaError_t e = cudaMemsetAsync(a.work, 0, kGradCounters * sizeof(int), s);
     if (e != cudaSuccess) return e;
     k_grad_setup<<<(a.n_flights + 127) / 128, 128, 0, s>>>(a);
-    e = launch_grad_forward(fwd, nsm, fwd_bps, s);
+    e = launch_grad_forward(fwd, nsm, fwd_bps, wide_bps, a.work + 4, s);
     if (e != cudaSuccess) return e;
     k_grad_order<<<1, kOrderThreads, 0, s>>>(a.steps, a.n_flights, a.order);
     if (mid) cudaEventRecord(mid, s);

@@ -54,6 +54,10 @@ struct FlightArgs {
     int* active_out;        // flights still airborne after this launch (nullptr: last launch)
     int* n_active_out;
     int* work;              // fetch counter, zero at launch
+    // pe_flight_quad.cu only: flights of the launch that have ended; once no more than hand_over are left
+    // a warp leaves its own to active_out (nullptr: never)
+    int* landed;
+    int hand_over;
     FlightState* state;     // [n_flights]
     float* dist;            // [n_flights] fitness per flight (metres; -100 oversize, -10 NaN)
     int* steps;             // [n_flights] integrated steps
@@ -100,13 +104,35 @@ size_t flight_smem_bytes(const FlightShape& sh);
 cudaError_t launch_flight(const FlightArgs& a, const FlightShape& sh, int grid, cudaStream_t s);
 int flight_fast_blocks_per_sm(const FlightShape& sh);
 cudaError_t launch_flight_fast(const FlightArgs& a, const FlightShape& sh, int grid, cudaStream_t s);
-// pe_grad's forward pass: the body-frame flight kernel with smoothed landing distances on the
-// gradient model's set-up (grad_setup), writing grad_ck, grad_fsum and grad_kind.  One launch over
-// every flight (step_begin 0, step_end = max_steps); 32 lanes per flight in 4-warp blocks for at
-// most 192 flights per SM, else the evaluation's one-warp shape.
+// Which kernels fly a batch in the default shape (results do not depend on it), by flights per SM.
+// Measured on GB300, milliseconds for pop x 8 with the launch's last 6 flights per SM handed over:
+//   flights per SM            8     14     27     37     54    108    431
+//   a block per flight     0.78   1.24   1.88   2.36   3.41   6.10   23.3
+//   32 lanes, hand-over    0.82   1.02   1.39   1.76   2.32   3.92      -
+//   four per warp, same    0.87   1.21   1.50     -    2.08   3.36   10.8
+// Hand-over at 2, 4, 8 and 12 flights per SM: 2.22, 2.07, 2.06, 2.10 ms at 54; none: 2.74.
+constexpr long long kWideFlights = 8;    // per SM: at most this many take a block each
+constexpr long long kLanesFlights = 32;  // at most this many 32 lanes each, more four per warp
+constexpr int kHandOver = 6;             // the last flights per SM go on with a block each
+constexpr long long kGradLanesFlights = 192;
+
+// The body-frame flight with four flights per warp and 48 per SM (pe_flight_quad.cu): evaluations of
+// many flights, one block per SM.  flight_quad_configure once per device before the first launch.
+cudaError_t flight_quad_configure();
+cudaError_t launch_flight_quad(const FlightArgs& a, int nsm, cudaStream_t s);
+// The body-frame flight with a block per flight (pe_flight_wide.cu): few flights, or few left.
+cudaError_t flight_wide_configure(int* bps);
+cudaError_t launch_flight_wide(const FlightArgs& a, int nsm, int bps, cudaStream_t s);
+// pe_grad's forward pass: the body-frame flight kernels with smoothed landing distances on the
+// gradient model's set-up (grad_setup), writing grad_ck, grad_fsum and grad_kind.  Over every flight
+// (step_begin 0, step_end = max_steps): a block per flight for at most kWideFlights per SM; 32 lanes
+// per flight in 4-warp blocks for at most kGradLanesFlights, handing the last ones over (a.landed,
+// a.hand_over, a.active_out, a.n_active_out; wide_work is the second queue's counter, zero at launch);
+// else the evaluation's one-warp shape.
 // Shared-memory opt-in and blocks per SM of its two shapes (32-lane, 16-lane), once per engine.
 cudaError_t grad_forward_configure(int bps[2]);
-cudaError_t launch_grad_forward(const FlightArgs& a, int nsm, const int bps[2], cudaStream_t s);
+cudaError_t launch_grad_forward(const FlightArgs& a, int nsm, const int bps[2], int wide_bps, int* wide_work,
+                                cudaStream_t s);
 cudaError_t launch_debug_step_fast(const FlightArgs& a, const FlightState* state_in, FlightState* state_out,
                                    float* FT, int* done, float* fit, int step, int lanes, cudaStream_t s);
 
@@ -132,6 +158,8 @@ constexpr int kAdjStride = 8 + 7 * kNtMax;
 constexpr int kGradMaxSeeds = 256;
 constexpr int kGradMaxK = 600;
 
+constexpr int kGradCounters = 5;
+
 struct GradArgs {
     const float4* pc;
     const float4* pn;
@@ -144,7 +172,8 @@ struct GradArgs {
     int K;                 // checkpoint interval (steps)
     int nck;               // checkpoints per flight: max_steps / K + 1
     int n_flights;         // pop * nseeds, flight f = p * nseeds + s
-    int* work;             // [2] queue counters (forward, reverse), zero at launch
+    int* work;             // [kGradCounters] queues (forward, reverse), flights ended and handed over by the
+                           // forward pass, its second queue; zeroed by launch_grad
     float* setup;          // [n_flights][kGradSetupFloats] the model's set-up of each flight
     float* ck;             // [n_flights][nck][16] checkpointed states
     float* fsum;           // [n_flights][max_steps][8] each step's body force and torque, written by
@@ -174,8 +203,8 @@ int grad_group_size(int K);
 // -> genome, on stream s.
 // With a.n_long > 0 the longest flights' reverse pass runs pipelined beside the others'; with
 // a.group > 1 the others run a.group flights per block.
-cudaError_t launch_grad(const GradArgs& a, const FlightArgs& fwd, int nsm, const int fwd_bps[2], const int rev_grid[2],
-                        cudaStream_t s, cudaEvent_t mid);
+cudaError_t launch_grad(const GradArgs& a, const FlightArgs& fwd, int nsm, const int fwd_bps[2], int wide_bps,
+                        const int rev_grid[2], cudaStream_t s, cudaEvent_t mid);
 // Whether checkpoint interval K admits the pipelined pass for the longest flights (K <= kPipeMaxK).
 bool grad_long_pass(int K);
 constexpr int kPipeMaxK = 96;

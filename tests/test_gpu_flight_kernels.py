@@ -1,0 +1,77 @@
+"""The kernels that the default shape chooses among (a block per flight, 32 lanes with a hand-over, four
+flights per warp) against the explicit 32-lane shape: one summation order, so every distance, step count
+and score is equal bit for bit, at the edges of each kernel's range."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _flights(torch, pe, G, seeds, shape=None, vary=0, max_steps=7200, smooth=0):
+    e = pe.Engine(0)
+    if shape:
+        e.set_config(**shape)
+    e.set_smooth_landing(smooth)
+    pop, n = G.shape[0], G.shape[0] * len(seeds)
+    g = torch.from_numpy(G).cuda()
+    dist = torch.full((n,), 7.0, device="cuda")
+    steps = torch.full((n,), -7, dtype=torch.int32, device="cuda")
+    scores = torch.empty(pop, device="cuda")
+    out = []
+    for _ in range(2):  # the second call finds the first one's lists and states
+        e.eval_batch(g, pop, seeds, vary, max_steps, dist, steps, scores)
+        torch.cuda.synchronize()
+        out.append([x.cpu().numpy().view(np.int32).copy() for x in (dist, steps, scores)])
+    e.close()
+    assert all(np.array_equal(a, b) for a, b in zip(*out))
+    return out[0]
+
+
+def _same(torch, pe, G, seeds, **kw):
+    want = _flights(torch, pe, G, seeds, shape=dict(lanes=32, warps=4, reg_cap=0, chunk=7200), **kw)
+    got = _flights(torch, pe, G, seeds, **kw)
+    for name, a, b in zip(("dist", "steps", "scores"), got, want):
+        assert np.array_equal(a, b), (name, int((a != b).sum()))
+
+
+@pytest.mark.parametrize("per_sm, extra", [(0, 1), (0, 3), (1, 0), (8, -1), (8, 0), (8, 1), (14, 5), (32, 0), (32, 1), (50, 7)])
+def test_default_kernels_at_their_edges(cuda, pe, oracle, per_sm, extra):
+    n = per_sm * cuda.cuda.get_device_properties(0).multi_processor_count + extra
+    G = oracle.grand(400 + n, n)
+    if n > 20:
+        G[3, 11] = np.nan  # nose ballast: flies one step and reports a NaN flight
+    _same(cuda, pe, G, [5])
+
+
+@pytest.mark.parametrize("max_steps", [1, 2, 8, 9, 16, 17, 599, 600, 601, 1300])
+@pytest.mark.parametrize("pop", [40, 300, 900])  # a block per flight, 32 lanes, four per warp
+def test_default_kernels_horizon(cuda, pe, oracle, pop, max_steps):
+    """Horizons about the polls for the hand-over and the clock's restart."""
+    _same(cuda, pe, oracle.grand(11, pop), [1, 2, 3, 4, 5, 6, 7], max_steps=max_steps)
+
+
+@pytest.mark.parametrize("pop", [40, 300, 900])
+@pytest.mark.parametrize("vary, smooth", [(1, 0), (0, 1)])
+def test_default_kernels_options(cuda, pe, oracle, pop, vary, smooth):
+    _same(cuda, pe, oracle.grand(12, pop), [3, 7922, 15841, 23760, 31679, -4, 9], vary=vary, smooth=smooth)
+
+
+@pytest.mark.parametrize("every", [1, 59, 60, 600])
+def test_gradient_forward_kernels(cuda, pe, oracle, every):
+    """The same genomes in a batch of a block per flight and in one that is handed over: distances and
+    objectives bit for bit, gradients to the reverse kernels' own 1e-5 of the norm."""
+    torch = cuda
+    G, seeds, out = oracle.grand(21, 240), list(range(1, 9)), []
+    for n in (20, 240):
+        e = pe.Engine(0)
+        g = torch.from_numpy(G[:n]).cuda()
+        grad, obj = torch.empty(n, 35, device="cuda"), torch.empty(n, device="cuda")
+        dist = torch.empty(n * 8, device="cuda")
+        e.grad(g, n, seeds, grad, max_steps=2400, checkpoint_every=every, d_obj=obj, d_dist=dist)
+        torch.cuda.synchronize()
+        out.append((dist[:160].cpu().numpy(), obj[:20].cpu().numpy(), grad[:20].cpu().numpy().astype(np.float64)))
+        e.close()
+    a, b = out
+    assert np.array_equal(a[0].view(np.int32), b[0].view(np.int32))
+    assert np.array_equal(a[1].view(np.int32), b[1].view(np.int32))
+    assert np.linalg.norm(a[2] - b[2]) <= 1e-5 * np.linalg.norm(b[2])
