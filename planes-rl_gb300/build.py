@@ -23,13 +23,13 @@ NVCC = os.environ.get("NVCC", "nvcc")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 CU_FLAGS = ["-O3", "-use_fast_math", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xptxas", "-warn-spills"]
 CU_SOURCES = ["pe_prepare.cu", "pe_flight.cu", "pe_flight_fast.cu", "pe_flight_quad.cu", "pe_flight_wide.cu", "pe_scores.cu", "pe_api.cu", "pe_probe.cu",
-              "pe_noalloc.cu", "pe_grad.cu", "pe_objective.cu", "pe_ga.cu", "pe_audit.cu"]
+              "pe_noalloc.cu", "pe_grad.cu", "pe_grad_time.cu", "pe_objective.cu", "pe_ga.cu", "pe_audit.cu"]
 # The gradient and the objective it differentiates are built without fast math: they are checked
 # against FP64 finite differences, and the FP64 objective must stay FP64.
-PRECISE_SOURCES = {"pe_grad.cu", "pe_objective.cu"}
+PRECISE_SOURCES = {"pe_grad.cu", "pe_grad_time.cu", "pe_objective.cu"}
 HOST_SOURCES = ["pe_host.cpp", "pe_drivers.cpp"]
 CLI_SOURCES = ["pe_cli.cpp"]
-HEADERS = ["pe_model.cuh", "pe_internal.cuh", "pe_grad_model.h", "pe_f32x2.cuh", "pe_flight_fast.cuh"]
+HEADERS = ["pe_model.cuh", "pe_internal.cuh", "pe_grad_model.h", "pe_f32x2.cuh", "pe_flight_fast.cuh", "pe_grad_common.cuh"]
 
 
 def _stale(out, deps):

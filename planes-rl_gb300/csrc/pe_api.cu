@@ -135,7 +135,8 @@ struct pe_engine {
     int wide_bps = 0;    // blocks per SM of the block-per-flight kernel, once both default kernels are set up
     // gradient
     DevBuf<float> g_setup, g_ck, g_adj, g_ybar, g_dist, g_fsum;
-    DevBuf<int> g_steps, g_kind, g_order, g_work;
+    DevBuf<float> g_rec, g_after;
+    DevBuf<int> g_steps, g_kind, g_order, g_work, g_items;
     int g_K = 0, g_rev_grid[2] = {0, 0}, g_fwd_bps[2] = {0, 0};
     // objective only
     DevBuf<double> o_plane, o_dist;
@@ -561,7 +562,6 @@ int pe_grad(pe_engine* e, const float* d_genomes, int pop, const int* h_seeds, i
     }
     PE_CUDA(e->g_setup.ensure((size_t)nf * kGradSetupFloats));
     PE_CUDA(e->g_ck.ensure((size_t)nf * nck * 16));
-    PE_CUDA(e->g_adj.ensure((size_t)nf * kAdjStride));
     PE_CUDA(e->g_ybar.ensure((size_t)pop * kAdjStride));
     PE_CUDA(e->g_steps.ensure((size_t)nf));
     PE_CUDA(e->g_kind.ensure((size_t)nf));
@@ -600,7 +600,6 @@ int pe_grad(pe_engine* e, const float* d_genomes, int pop, const int* h_seeds, i
     a.steps = e->g_steps.p;
     a.kind = e->g_kind.p;
     a.order = e->g_order.p;
-    a.adj = e->g_adj.p;
     a.ybar = e->g_ybar.p;
     a.obj = d_obj;
     a.grad = d_grad;
@@ -627,28 +626,55 @@ int pe_grad(pe_engine* e, const float* d_genomes, int pop, const int* h_seeds, i
         fa.active_out = e->list0.p;
         fa.n_active_out = a.work + 3;
     }
-    // The reverse pass is bound by its longest flights' chains and by how many flights it keeps in
-    // flight.  With the stored forces the flights other than the longest take grad_group_size(K) per
-    // block, warp 0 carrying all their integrator chains at once: the longest take the pipelined
-    // pass (one per 8 SMs, one per 4 SMs in a batch of at most 4 flights per SM such as the GA's
-    // polish of 64 genomes x 8 scenarios), the next nsm a block each, the rest shared.  Measured at
-    // 256 x 8: 4.45 ms per call with one flight per block, 3.9 ms so; at 64 x 8: 2.76 and 2.67 ms.
-    // Which flights share a block changes no bit of the result.  PE_GRAD_GROUP in the environment:
-    // 1 gives every flight a block of its own in that kernel, 0 takes the one-flight kernel (the
-    // same gradients to ~1e-6, its panel sums running over 4 warps instead of 3; it takes the
-    // pipelined pass only in a small batch, as at 256 x 8 that gains it nothing).
+    // The serial reverse kernels are bound by their longest flights' chains and by how many flights they
+    // keep in flight.  With the stored forces the flights other than the longest take grad_group_size(K)
+    // per block, warp 0 carrying all their integrator chains at once: the longest take the pipelined
+    // pass (one per 8 SMs, one per 4 SMs in a batch of at most 4 flights per SM), the next nsm a block
+    // each, the rest shared.  Which flights share a block changes no bit of the result.
     const char* group_env = getenv("PE_GRAD_GROUP");
     const int group_req = group_env ? atoi(group_env) : -1;
-    a.group = store_forces && group_req != 0 ? grad_group_size(K) : 1;
-    const bool small = nf <= 4 * e->nsm;
-    if (store_forces && grad_long_pass(K) && (small || a.group > 1))
-        a.n_long = std::min(nf, std::max(1, a.group > 1 && small ? e->nsm / 4 : e->nsm / 8));
-    a.n_single = a.group > 1 ? (group_req == 1 ? nf : e->nsm) : 0;
+    // The reverse pass parallel in time keeps records of every flight-step.  Where those do not fit
+    // kAdjBytes, or cannot be had, the serial kernels run, as with PE_GRAD_GROUP = 0 (one flight per
+    // block) or 2 (shared blocks).  PE_GRAD_STEPS in the environment lowers kAdjSteps: longer flights
+    // take the one-flight kernel (gradients within ~1e-6).  Measured at 256 x 8: 4.03 ms per call with
+    // the serial kernels, 3.32 ms so; at 64 x 8: 2.63 and 1.63 ms.
+    const char* steps_env = getenv("PE_GRAD_STEPS");
+    const int want_steps = steps_env ? std::max(1, std::min(kAdjSteps, atoi(steps_env))) : kAdjSteps;
+    const int rec_steps = (std::min(want_steps, max_steps) + 31) / 32 * 32;
+    const size_t rec_floats = (size_t)nf * ((size_t)rec_steps * kAdjEnt + (size_t)(rec_steps / 32) * kAdjChunk);
+    const int parts = (rec_steps + kAdjPart - 1) / kAdjPart;
+    if (store_forces && group_req != 0 && group_req != 2 && rec_floats * sizeof(float) <= kAdjBytes) {
+        if (e->g_rec.ensure(rec_floats) == cudaSuccess && e->g_after.ensure((size_t)nf * 16) == cudaSuccess &&
+            e->g_items.ensure(grad_time_items(nf, rec_steps)) == cudaSuccess &&
+            e->g_adj.ensure((size_t)nf * parts * kAdjStride) == cudaSuccess) {
+            a.rec = e->g_rec.p;
+            a.rec_steps = rec_steps;
+            a.adj_parts = parts;
+            a.after = e->g_after.p;
+            a.items = e->g_items.p;
+            a.group = 1;
+        } else {
+            (void)cudaGetLastError();  // not an error of this call
+            e->g_rec.release();
+        }
+    }
+    if (!a.rec) {
+        a.adj_parts = 1;
+        PE_CUDA(e->g_adj.ensure((size_t)nf * kAdjStride));
+    }
+    a.adj = e->g_adj.p;
+    if (!a.rec) {
+        a.group = store_forces && group_req != 0 ? grad_group_size(K) : 1;
+        const bool small = nf <= 4 * e->nsm;
+        if (store_forces && grad_long_pass(K) && (small || a.group > 1))
+            a.n_long = std::min(nf, std::max(1, a.group > 1 && small ? e->nsm / 4 : e->nsm / 8));
+        a.n_single = a.group > 1 ? e->nsm : 0;
+    }
     PE_CUDA(launch_grad(a, fa, e->nsm, e->g_fwd_bps, e->wide_bps, e->g_rev_grid, s, e->ev[2]));
     PE_CUDA(record_event(e->ev[3], s));
-    // prepare (3), set-up, forward (two kernels with the hand-over), order, reverse (two with the
-    // pipelined pass), weights, genome
-    e->last_launches = 3 + 6 + (hand_over && nf > kWideFlights * e->nsm ? 1 : 0) + (a.n_long > 0 ? 1 : 0);
+    // prepare (3), set-up, forward (two kernels with the hand-over), order, reverse (five kernels parallel
+    // in time, two with the pipelined pass), weights, genome
+    e->last_launches = 3 + 6 + (hand_over && nf > kWideFlights * e->nsm ? 1 : 0) + (a.rec ? 4 + (max_steps > rec_steps) : a.n_long > 0);
     e->prepared_pop = pop;
     e->timed = true;
     return PE_OK;

@@ -11,12 +11,14 @@
 // Pipeline on one stream, after prepare (pe_prepare.cu) has written the plane table and panels:
 //   k_grad_setup    thread per flight: this model's print variation, scenario and release, as a
 //                   record for the forward pass.
-//   forward         the evaluation's body-frame flight kernel (pe_flight_fast.cu, its GRAD
-//                   instance) on those records: packed f32x2 panel pairs, smoothed distance, step
+//   forward         the evaluation's body-frame flight kernels (the GRAD instances of
+//                   pe_flight_fast.cu and pe_flight_wide.cu) on those records: packed f32x2 panel pairs, smoothed distance, step
 //                   count, how the flight ended, the state every K steps and every step's
 //                   body-frame force and torque.
 //   k_grad_order    one block: flights sorted by step count, longest first (counting sort), so
 //                   the reverse pass starts its longest flights first.
+//   reverse         the pass parallel in time (pe_grad_time.cu); where its records do not fit, the
+//                   serial kernels of this file:
 //   k_grad_reverse  a block of W warps per flight in that order: per segment of K steps (last
 //                   first) the states are rebuilt from the checkpoint through this model's
 //                   integrator on the forward's stored forces (or, when those were not kept, its
@@ -36,6 +38,7 @@
 #include <cstddef>
 
 #include "pe_f32x2.cuh"
+#include "pe_grad_common.cuh"
 #include "pe_grad_model.h"
 #include "pe_internal.cuh"
 
@@ -55,74 +58,6 @@
 namespace pe {
 
 namespace {
-
-using F3 = pg::V3<float>;
-using FSt = pg::St<float>;
-
-constexpr int kPanelFloats = 7 * kNtMax;  // rbx rby rbz nbx nby nbz ak (SoA)
-constexpr int kSegFloats = 20;            // state (14) + body force (3) + body torque (3)
-constexpr int kCkFloats = 16;             // one checkpointed state
-
-__device__ __forceinline__ float warp_sum(float v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-__device__ __forceinline__ FSt zero_state() {
-    FSt z;
-    z.pos = pg::v3(0.f, 0.f, 0.f);
-    z.vel = z.pos;
-    z.w = z.pos;
-    z.q[0] = z.q[1] = z.q[2] = z.q[3] = 0.f;
-    z.t = 0.f;
-    return z;
-}
-
-// Constants of one flight: scenario draw, print variation, gust phase.
-struct FlightCtx {
-    pg::FlightP<float> P;
-    F3 cg;
-    float sigma, beta[6];
-    float sc[kScenN];
-    int nt, off;
-};
-
-__device__ __forceinline__ void flight_setup(const GradArgs& a, int f, FlightCtx& c) {
-    const int p = f / a.nseeds, s = f - p * a.nseeds;
-    const int seed = a.seeds[s] + (a.vary ? p * 7919 : 0);
-    Scenario S;
-    scenario_desc(seed, &S);
-#pragma unroll
-    for (int k = 0; k < kScenN; k++) c.sc[k] = S.v[k];
-    const float* mp = a.plane_mp + (size_t)p * kMpN;
-    float I[6];
-#pragma unroll
-    for (int k = 0; k < 6; k++) I[k] = mp[5 + k];
-    pg::printed(c.sc, mp[0], I, c.P, &c.cg, &c.sigma, c.beta);
-    c.P.phase = seed_phase(seed);
-    c.nt = a.plane_nt[p];
-    c.off = a.plane_off[p];
-}
-
-// A flight's constants as k_grad_setup wrote them: the forward pass flew with these, and every
-// reverse kernel takes them from here rather than from its own flight_setup, whose rounding may
-// differ in the last place with how the compiler fuses it into each kernel.
-__device__ __forceinline__ pg::FlightP<float> setup_flightp(const GradArgs& a, int f) {
-    const float* r = a.setup + (size_t)f * kGradSetupFloats;
-    pg::FlightP<float> P;
-    P.mass = r[0];
-    P.invmass = r[1];
-#pragma unroll
-    for (int k = 0; k < 6; k++) P.I[k] = r[2 + k];
-#pragma unroll
-    for (int k = 0; k < 9; k++) P.invI[k] = r[8 + k];
-    P.cf = r[17];
-    P.phase = r[18];
-    P.gust = r[19];
-    P.base_x = r[20];
-    P.base_y = r[21];
-    return P;
-}
 
 // Print-warped body-frame panels of one flight into shared memory (SoA), by all nthr threads.
 __device__ __forceinline__ void stage_panels(const GradArgs& a, const FlightCtx& c, float* sp, int tid, int nthr) {
@@ -173,36 +108,6 @@ __device__ __forceinline__ void panel_partial_nt(const pg::Pre<float>& pr, const
     else panel_partial<PPT>(pr, sp, nt, cf, tid, nthr, out);
 }
 
-__device__ __forceinline__ void store_state16(float* dst, const FSt& s) {
-    float4* d4 = reinterpret_cast<float4*>(dst);
-    d4[0] = make_float4(s.pos.x, s.pos.y, s.pos.z, s.q[0]);
-    d4[1] = make_float4(s.q[1], s.q[2], s.q[3], s.vel.x);
-    d4[2] = make_float4(s.vel.y, s.vel.z, s.w.x, s.w.y);
-    d4[3] = make_float4(s.w.z, s.t, 0.f, 0.f);
-}
-__device__ __forceinline__ FSt load_state16(const float* src) {
-    const float4* s4 = reinterpret_cast<const float4*>(src);
-    const float4 a = s4[0], b = s4[1], c = s4[2], d = s4[3];
-    FSt s;
-    s.pos = pg::v3(a.x, a.y, a.z);
-    s.q[0] = a.w; s.q[1] = b.x; s.q[2] = b.y; s.q[3] = b.z;
-    s.vel = pg::v3(b.w, c.x, c.y);
-    s.w = pg::v3(c.z, c.w, d.x);
-    s.t = d.y;
-    return s;
-}
-// A step's body force and torque as the forward pass stores them (2 float4).
-__device__ __forceinline__ void store_fsum(float* dst, F3 F, F3 T) {
-    float4* d4 = reinterpret_cast<float4*>(dst);
-    d4[0] = make_float4(F.x, F.y, F.z, T.x);
-    d4[1] = make_float4(T.y, T.z, 0.f, 0.f);
-}
-__device__ __forceinline__ void load_fsum(const float* src, F3* F, F3* T) {
-    const float4* s4 = reinterpret_cast<const float4*>(src);
-    const float4 a = s4[0], b = s4[1];
-    *F = pg::v3(a.x, a.y, a.z);
-    *T = pg::v3(a.w, b.x, b.y);
-}
 // Segment entry: the state before a step and that step's body force and torque (5 float4).
 __device__ __forceinline__ void store_seg(float* dst, const FSt& s, F3 F, F3 T) {
     float4* d4 = reinterpret_cast<float4*>(dst);
@@ -232,9 +137,6 @@ __device__ __forceinline__ FSt load_seg(const float* src, F3* F, F3* T) {
 //   [0..13] pos q vel w t  [14..16] Fb  [17..19] Tb  [20..22] va  [23..25] vb  [26..34] J
 //   [35..37] Fw  [38..40] Iw  [41..43] tq  [44..46] w1  [47..49] wn  [50..52] vel1  [53..56] qo  [57] il
 constexpr int kEntFloats = 60;
-
-__device__ __forceinline__ void put3(float* d, F3 v) { d[0] = v.x; d[1] = v.y; d[2] = v.z; }
-__device__ __forceinline__ F3 get3(const float* d) { return pg::v3(d[0], d[1], d[2]); }
 
 // The integrator's part of an entry (state, forces, intermediates), written by one lane.
 __device__ __forceinline__ void put_entry_post(float* e, const FSt& s, F3 Fb, F3 Tb, const pg::PostF<float>& f) {
@@ -583,7 +485,8 @@ __global__ void __launch_bounds__(32 * W, LONG ? 1 : (W >= 8 ? 1 : 12 / W)) k_gr
         }
         if (idx >= (LONG ? a.n_long : a.n_flights)) break;
         const int f = a.order[idx];
-        float* out = a.adj + (size_t)f * kAdjStride;
+        if (!LONG && a.rec && a.steps[f] <= a.rec_steps) break;  // these and all later ones went parallel in time
+        float* out = a.adj + (size_t)f * a.adj_parts * kAdjStride;
         const int kind = a.kind[f];
         if (kind == 0 || kind == 3) {  // oversize or NaN flight: constant distance
             for (int i = tid; i < kAdjStride; i += nthr) out[i] = 0.f;
@@ -925,42 +828,7 @@ struct GroupShared {
     int rchunk[M];          // pipelined: steps to the next 600-step clock restart
 };
 
-// An entry of the pipelined grouped pass (kPEnt floats): the state before a step, the step's body
-// force and torque (written by the rebuild) and its step_pre values (written one iteration later):
-//   [0..13] pos q vel w t  [16..18] Fb  [19..21] Tb  [24..26] va  [28..30] vb
-//   the gust Jacobian J (row-major) in the gaps [14] [15] [22] [23] [27] [31] [32] [33] [34]
-constexpr int kPEnt = 36;
 constexpr int kPipeGroupMaxK = 60;  // one segment of entries per flight: 4 blocks of 3 warps per SM
-__device__ __forceinline__ void put_pent_post(float* e, const FSt& s, F3 F, F3 T) {
-    store_state16(e, s);
-    store_fsum(e + 16, F, T);
-}
-__device__ __forceinline__ void put_pent_pre(float* e, const pg::Pre<float>& q, const float (*J)[3]) {
-    e[14] = J[0][0]; e[15] = J[0][1]; e[22] = J[0][2];
-    e[23] = J[1][0]; e[27] = J[1][1]; e[31] = J[1][2];
-    e[32] = J[2][0]; e[33] = J[2][1]; e[34] = J[2][2];
-    put3(e + 24, q.va);
-    put3(e + 28, q.vb);
-}
-__device__ __forceinline__ void get_pent(const float* e, FSt& s, F3* F, F3* T, pg::Pre<float>& q, float (*J)[3]) {
-    const float4* e4 = reinterpret_cast<const float4*>(e);
-    const float4 a = e4[0], b = e4[1], c = e4[2], d = e4[3], f0 = e4[4], f1 = e4[5], v0 = e4[6], v1 = e4[7],
-                 j2 = e4[8];
-    s.pos = pg::v3(a.x, a.y, a.z);
-    s.q[0] = a.w; s.q[1] = b.x; s.q[2] = b.y; s.q[3] = b.z;
-    s.vel = pg::v3(b.w, c.x, c.y);
-    s.w = pg::v3(c.z, c.w, d.x);
-    s.t = d.y;
-    J[0][0] = d.z; J[0][1] = d.w;
-    *F = pg::v3(f0.x, f0.y, f0.z);
-    *T = pg::v3(f0.w, f1.x, f1.y);
-    J[0][2] = f1.z; J[1][0] = f1.w;
-    q.va = pg::v3(v0.x, v0.y, v0.z);
-    J[1][1] = v0.w;
-    q.vb = pg::v3(v1.x, v1.y, v1.z);
-    J[1][2] = v1.w;
-    J[2][0] = j2.x; J[2][1] = j2.y; J[2][2] = j2.z;
-}
 template <int W, int M>
 __host__ __device__ constexpr int group_head_floats() { return (int)((sizeof(GroupShared<W, M>) + 15) / 16 * 4); }
 
@@ -1023,7 +891,7 @@ __global__ void __launch_bounds__(32 * W, (W >= 8 ? 1 : 12 / W)) k_grad_reverse_
         for (int m = 0; m < M; m++) {
             const int f = sh.f[m];
             if (f < 0) continue;
-            float* out = a.adj + (size_t)f * kAdjStride;
+            float* out = a.adj + (size_t)f * a.adj_parts * kAdjStride;
             if (sh.k[m] < 0) {
                 for (int i = tid; i < kAdjStride; i += nthr) out[i] = 0.f;
                 continue;
@@ -1362,27 +1230,38 @@ __global__ void __launch_bounds__(32 * W, (W >= 8 ? 1 : 12 / W)) k_grad_reverse_
 // ------------------------------------------------------------------ per plane: weights and genome contraction
 // Tail weights of a plane's distances and the weighted sum of its flights' adjoints (ybar).
 constexpr int kWeightThreads = 128;
+constexpr int kWeightSplit = 8;  // blocks per plane: a thread's sums are chains of loads (1 block: 110 us at 256 x 8)
 __global__ void __launch_bounds__(kWeightThreads) k_grad_weights(GradArgs a) {
     __shared__ float w[kGradMaxSeeds], d[kGradMaxSeeds];
+    __shared__ int parts[kGradMaxSeeds];  // records of each flight's adjoints
     __shared__ float J;
     const int p = blockIdx.x, tid = threadIdx.x, S = a.nseeds;
     const int nt = a.plane_nt[p];
     float* yb = a.ybar + (size_t)p * kAdjStride;
     if (nt <= 0) {  // oversize: the objective is the constant -100
-        if (tid == 0 && a.obj) a.obj[p] = -100.f;
+        if (tid == 0 && blockIdx.y == 0 && a.obj) a.obj[p] = -100.f;
         return;
     }
-    for (int s = tid; s < S; s += kWeightThreads) d[s] = a.dist[(size_t)p * S + s];
+    for (int s = tid; s < S; s += kWeightThreads) {
+        const int f = p * S + s, kind = a.kind[f], n = a.steps[f];
+        d[s] = a.dist[f];
+        parts[s] = a.rec && (kind == 1 || kind == 2) && n <= a.rec_steps ? (n + kAdjPart - 1) / kAdjPart : 1;
+    }
     __syncthreads();
     if (tid == 0) J = pg::objective_weights(d, S, w);
     __syncthreads();
-    if (tid == 0 && a.obj) a.obj[p] = J;
-    const float* base = a.adj + (size_t)p * S * kAdjStride;
-    for (int i = tid; i < 8 + 7 * nt; i += kWeightThreads) {
+    if (tid == 0 && blockIdx.y == 0 && a.obj) a.obj[p] = J;
+    const float* base = a.adj + (size_t)p * S * a.adj_parts * kAdjStride;
+    for (int i = blockIdx.y * kWeightThreads + tid; i < 8 + 7 * nt; i += kWeightThreads * gridDim.y) {
         // entries 0..7 (mass, I, pad), then 7 panel fields of nt each at stride kNtMax
         const int q = i < 8 ? i : 8 + ((i - 8) / nt) * kNtMax + (i - 8) % nt;
         float acc = 0.f;
-        for (int s = 0; s < S; s++) acc += w[s] * base[(size_t)s * kAdjStride + q];
+        for (int s = 0; s < S; s++) {
+            const float* r = base + (size_t)s * a.adj_parts * kAdjStride + q;
+            float x = r[0];
+            for (int i = 1; i < parts[s]; i++) x += r[(size_t)i * kAdjStride];
+            acc += w[s] * x;
+        }
         yb[q] = acc;
     }
 }
@@ -1534,7 +1413,7 @@ cudaError_t grad_configure(int K, int rev_grid[2], int nsm) {
 cudaError_t launch_grad(const GradArgs& a, const FlightArgs& fwd, int nsm, const int fwd_bps[2], int wide_bps,
                         const int rev_grid[2], cudaStream_t s, cudaEvent_t mid) {
     const bool grouped = a.group > 1;
-    if (grouped && (a.group != kRevGroup || !a.fsum || rev_grid[1] <= 0)) return cudaErrorInvalidValue;
+    if (grouped && !a.rec && (a.group != kRevGroup || !a.fsum || rev_grid[1] <= 0)) return cudaErrorInvalidValue;
     cudaError_t e = cudaMemsetAsync(a.work, 0, kGradCounters * sizeof(int), s);
     if (e != cudaSuccess) return e;
     k_grad_setup<<<(a.n_flights + 127) / 128, 128, 0, s>>>(a);
@@ -1542,7 +1421,12 @@ cudaError_t launch_grad(const GradArgs& a, const FlightArgs& fwd, int nsm, const
     if (e != cudaSuccess) return e;
     k_grad_order<<<1, kOrderThreads, 0, s>>>(a.steps, a.n_flights, a.order);
     if (mid) cudaEventRecord(mid, s);
-    if (a.n_long > 0) {
+    if (a.rec) {
+        e = launch_grad_time(a, nsm, s);
+        if (e != cudaSuccess) return e;
+        if (a.max_steps > a.rec_steps)
+            k_grad_reverse<kRevW, kSolo, false><<<rev_grid[0], 32 * kRevW, grad_reverse_smem(a.K), s>>>(a);
+    } else if (a.n_long > 0) {
         // the longest flights' pipelined pass first; the other flights' kernel is its programmatic
         // dependent, so it starts once those blocks are resident and fills the rest of the GPU
         k_grad_reverse<kRevW, kSolo, true><<<a.n_long, 32 * kRevW, grad_reverse_long_smem(a.K), s>>>(a);
@@ -1570,7 +1454,7 @@ cudaError_t launch_grad(const GradArgs& a, const FlightArgs& fwd, int nsm, const
     } else {
         k_grad_reverse<kRevW, kSolo, false><<<rev_grid[0], 32 * kRevW, grad_reverse_smem(a.K), s>>>(a);
     }
-    k_grad_weights<<<a.pop, kWeightThreads, 0, s>>>(a);
+    k_grad_weights<<<dim3(a.pop, kWeightSplit), kWeightThreads, 0, s>>>(a);
     k_grad_genome<<<a.pop * kGenomeN, kGenomeThreads, 0, s>>>(a);
     return cudaGetLastError();
 }

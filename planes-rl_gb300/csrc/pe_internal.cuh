@@ -158,7 +158,13 @@ constexpr int kAdjStride = 8 + 7 * kNtMax;
 constexpr int kGradMaxSeeds = 256;
 constexpr int kGradMaxK = 600;
 
-constexpr int kGradCounters = 5;
+constexpr int kGradCounters = 9;
+// The reverse pass parallel in time (pe_grad_time.cu) keeps an entry per flight-step and a chunk of
+// matrices per 32 of them, for flights of at most kAdjSteps steps, and adds the plane's adjoints in parts
+// of kAdjPart steps; it is taken where the records fit kAdjBytes.
+constexpr int kAdjEnt = 24, kAdjChunk = 4292;
+constexpr int kAdjSteps = 3072, kAdjPart = 512;
+constexpr size_t kAdjBytes = 8ull << 30;
 
 struct GradArgs {
     const float4* pc;
@@ -173,7 +179,8 @@ struct GradArgs {
     int nck;               // checkpoints per flight: max_steps / K + 1
     int n_flights;         // pop * nseeds, flight f = p * nseeds + s
     int* work;             // [kGradCounters] queues (forward, reverse), flights ended and handed over by the
-                           // forward pass, its second queue; zeroed by launch_grad
+                           // forward pass, its second queue, count and queue of the Jacobians' and of the
+                           // panels' items; zeroed by launch_grad
     float* setup;          // [n_flights][kGradSetupFloats] the model's set-up of each flight
     float* ck;             // [n_flights][nck][16] checkpointed states
     float* fsum;           // [n_flights][max_steps][8] each step's body force and torque, written by
@@ -186,7 +193,13 @@ struct GradArgs {
     int group;             // flights per block of the other flights' reverse pass: 1, or
                            // grad_group_size(K) with fsum
     int n_single;          // grouped: the first n_single flights after the n_long take a block each
-    float* adj;            // [n_flights][kAdjStride]
+    float* adj;            // [n_flights][adj_parts][kAdjStride]
+    // the reverse pass parallel in time (rec null: the serial kernels)
+    float* rec;            // entries [n_flights][rec_steps][kAdjEnt], then chunks [n_flights][rec_steps / 32][kAdjChunk]
+    int rec_steps;         // flights of more steps take the serial kernel
+    int adj_parts;         // records per flight in adj
+    float* after;          // [n_flights][16] the state after the last step, then the release state's adjoint
+    int* items;            // [grad_time_items] work lists
     float* ybar;           // [pop][kAdjStride] weighted sum of each plane's flight adjoints
     float* obj;            // [pop] objective (may be null)
     float* grad;           // [pop][35]
@@ -205,6 +218,9 @@ int grad_group_size(int K);
 // a.group > 1 the others run a.group flights per block.
 cudaError_t launch_grad(const GradArgs& a, const FlightArgs& fwd, int nsm, const int fwd_bps[2], int wide_bps,
                         const int rev_grid[2], cudaStream_t s, cudaEvent_t mid);
+// The reverse pass parallel in time, from k_grad_order to the flights' adjoints.
+size_t grad_time_items(int n_flights, int rec_steps);
+cudaError_t launch_grad_time(const GradArgs& a, int nsm, cudaStream_t s);
 // Whether checkpoint interval K admits the pipelined pass for the longest flights (K <= kPipeMaxK).
 bool grad_long_pass(int K);
 constexpr int kPipeMaxK = 96;

@@ -75,3 +75,35 @@ def test_gradient_forward_kernels(cuda, pe, oracle, every):
     assert np.array_equal(a[0].view(np.int32), b[0].view(np.int32))
     assert np.array_equal(a[1].view(np.int32), b[1].view(np.int32))
     assert np.linalg.norm(a[2] - b[2]) <= 1e-5 * np.linalg.norm(b[2])
+
+
+@pytest.mark.parametrize("knob, value", [("PE_GRAD_GROUP", "2"), ("PE_GRAD_GROUP", "0"), ("PE_GRAD_STEPS", "300"),
+                                         ("PE_GRAD_STEPS", "1"), ("PE_GRAD_STEPS", "511"), ("PE_GRAD_STEPS", "513")])
+@pytest.mark.parametrize("pop, nseeds, max_steps, every", [(1, 1, 1, 1), (5, 3, 31, 7), (33, 5, 33, 60), (40, 8, 513, 60),
+                                                           (60, 4, 2400, 600)])
+def test_gradient_parallel_in_time(cuda, pe, oracle, monkeypatch, pop, nseeds, max_steps, every, knob, value):
+    """The reverse pass parallel in time against the serial kernels, and with its longer flights left to
+    them: objectives and distances bit for bit, each genome's gradient to 1e-5 of its norm (two float
+    adjoints of one trajectory; the serial kernels differ among themselves by 1e-6).  Horizons about its
+    chunks of 32 steps and its parts of 512."""
+    torch = cuda
+    G = oracle.grand(31, pop)
+    if pop > 4:
+        G[2, 11] = np.nan
+    e = pe.Engine(0)
+    g, out = torch.from_numpy(G).cuda(), []
+    for i in range(2):
+        if i:
+            monkeypatch.setenv(knob, value)
+        grad, obj = torch.full((pop, 35), 3.0, device="cuda"), torch.empty(pop, device="cuda")
+        dist = torch.empty(pop * nseeds, device="cuda")
+        e.grad(g, pop, list(range(1, nseeds + 1)), grad, max_steps=max_steps, checkpoint_every=every, d_obj=obj, d_dist=dist)
+        torch.cuda.synchronize()
+        out.append((dist.cpu().numpy(), obj.cpu().numpy(), grad.cpu().numpy().astype(np.float64)))
+    e.close()
+    a, b = out
+    assert np.array_equal(a[0].view(np.int32), b[0].view(np.int32)) and np.array_equal(a[1].view(np.int32), b[1].view(np.int32))
+    bad = np.isnan(b[2]).any(axis=1)  # the NaN genome's row: its zero adjoints times a NaN mesh, on either side
+    assert np.array_equal(np.isnan(a[2]), np.isnan(b[2])) and bad.sum() <= 1
+    norm = np.linalg.norm(b[2][~bad], axis=1)
+    assert (np.linalg.norm((a[2] - b[2])[~bad], axis=1) <= 1e-5 * norm).all()
