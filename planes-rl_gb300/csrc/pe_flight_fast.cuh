@@ -219,6 +219,9 @@ __device__ __forceinline__ void fast_rows(quat4 q, vec3* r0, vec3* r1, vec3* r2)
     *r2 = mk3(mul_(2.0f, sub_(xz, wy)), mul_(2.0f, add_(yz, wx)), fma_(-2.0f, add_(xx, yy), 1.0f));
 }
 
+// Packed constants as constant-bank operands: 1.9 (PE_CN_SLOPE), 1e-30 and -1, each twice.  As
+// immediates every use takes two moves into a register pair (28 of a flight-step's 400 instructions).
+static __constant__ unsigned long long c_k19 = 0x3ff333333ff33333ull, c_tiny = 0x0da242600da24260ull, c_mone = 0xbf800000bf800000ull;
 // Per-step constants of the packed panel pass (both halves equal).
 struct PairConst {
     f2 vbx, vby, vbz;     // body-frame air velocity
@@ -257,7 +260,7 @@ __device__ __forceinline__ void pair_force(f2 rbx, f2 rby, f2 rbz, f2 ak, f2 nbx
     upk(fma2(s, s, k.mone), ua, ub);
     const f2 sq = pk(sqrtf(fmaxf(0.0f, -ua)), sqrtf(fmaxf(0.0f, -ub)));
     // cn - cf s = s (1.9 sqrt(1 - s^2) + 2 |s| - cf)
-    const f2 g = fma2(k.k19, sq, pk(__fmaf_rn(2.0f, fabsf(sa), -k_cf_scalar), __fmaf_rn(2.0f, fabsf(sb), -k_cf_scalar)));
+    const f2 g = fma2(sq, k.k19, pk(__fmaf_rn(2.0f, fabsf(sa), -k_cf_scalar), __fmaf_rn(2.0f, fabsf(sb), -k_cf_scalar)));
     // -f = na nb + nb_ vr with na = qd (cn - cf s), nb_ = qd cf / |vr|
     const f2 na = mul2(mul2(qd, s), g);
     const f2 nv = mul2(mul2(qd, k.cf), inv);
@@ -366,11 +369,14 @@ __device__ __forceinline__ vec3 fast_body(vec3 r0, vec3 r1, vec3 r2, vec3 v) {
                fma_(r2.z, v.z, fma_(r1.z, v.y, mul_(r0.z, v.x))));
 }
 
-__device__ __forceinline__ StepPre fast_pre(const FastConst& fc, FlightState& st, int step) {
+// LANES: the gusts with one sine per lane (wl, of lane i mod 8 of the flight).
+template <bool LANES = false>
+__device__ __forceinline__ StepPre fast_pre(const FastConst& fc, FlightState& st, int step, const WindLane* wl = nullptr) {
     if (step > 0 && step % kChunk == 0) st.t = mul_((float)step, PE_DT);
     StepPre pre;
     fast_rows(st.q, &pre.r0, &pre.r1, &pre.r2);
-    const vec3 wind = fast_wind(st.pos, st.t, fc.phase, fc.gust, fc.base_x, fc.base_y);
+    const vec3 wind = LANES ? wind_lanes(st.pos, mul_(wl->ct, st.t), *wl, fc.gust, fc.base_x, fc.base_y)
+                            : fast_wind(st.pos, st.t, fc.phase, fc.gust, fc.base_x, fc.base_y);
     const vec3 va = mk3(sub_(st.vel.x, wind.x), sub_(st.vel.y, wind.y), sub_(st.vel.z, wind.z));
     pre.vb = fast_body(pre.r0, pre.r1, pre.r2, va);
     return pre;
@@ -381,7 +387,7 @@ __device__ __forceinline__ PairConst pair_const(const FastConst& fc, vec3 vb, ve
     k.vbx = bc(vb.x); k.vby = bc(vb.y); k.vbz = bc(vb.z);
     k.wbx = bc(wb.x); k.wby = bc(wb.y); k.wbz = bc(wb.z);
     k.nwbx = bc(-wb.x); k.nwby = bc(-wb.y); k.nwbz = bc(-wb.z);
-    k.k19 = bc(PE_CN_SLOPE); k.cf = bc(fc.skin_cf); k.tiny = bc(1e-30f); k.mone = bc(-1.0f);
+    k.k19 = c_k19; k.cf = bc(fc.skin_cf); k.tiny = c_tiny; k.mone = c_mone;
     return k;
 }
 

@@ -7,7 +7,7 @@
 // without a ready one.  Here a warp flies four flights: it evaluates their panels one flight after the
 // other on all 32 lanes, reduces the four sets of sums in one transposed tree that leaves flight g's
 // totals on lanes 8g..8g+7, and those eight lanes integrate it, so one instruction stream carries four
-// scalar parts (402 instructions per flight-step, and planes of 88 and 172 pairs no longer share a
+// scalar parts (358 instructions per flight-step, and planes of 88 and 172 pairs no longer share a
 // warp's pass count).
 //
 // Room for 48 flights per SM (12 warps) instead of 22 comes from tensor memory: a lane always reads
@@ -18,11 +18,13 @@
 // registers to the panel part (136 of them, no spills).
 //
 // Bound: register reads.  A packed FMA of three register operands reads six registers through two
-// banks, three cycles instead of the pipe's two; per flight-step 172 packed and 78 scalar FMA-pipe
-// instructions take 646 cycles of a scheduler (420 by pipe rate, 585 by reads).  16 warps of three
+// banks, three cycles instead of the pipe's two; per flight-step 172 packed and 67 scalar FMA-pipe
+// instructions take 592 cycles of a scheduler (411 by pipe rate, about 540 by reads).  16 warps of three
 // flights (128 registers) took 203.9 ms where 12 of four took 189.3, so more warps do not help.
 // Measured, 100,000 x 12 flights: 218.3 ms a flight per half warp, 195.2 four per warp with the state in
-// registers, 189.3 in shared memory, 184.1 with warp-uniform control flow and the hand-over.
+// registers, 189.3 in shared memory, 184.5 with warp-uniform control flow and the hand-over, 174.4 with
+// the four flights' code unrolled (no copies between the folds), 173.0 with the packed constants in the
+// constant bank, 172.1 with a gust sine per lane.
 //
 // The sums run in the fixed order of pe_flight_fast.cuh, so every distance and step count is
 // bit-identical to the other kernels'.
@@ -117,7 +119,7 @@ __device__ __forceinline__ f2 word2(const TmWords& x, int i) {
 
 // A value that all lanes hold.  Every branch around the panel part hangs on such values, so that the
 // compiler can prove the warp converged there and use the uniform datapath for its addresses
-// (186.3 to 184.9 ms at 100,000 x 12).
+// and the step's rates (186.3 to 184.9 ms at 100,000 x 12; loaded as packed pairs instead: 176.3 to 174.4).
 __device__ __forceinline__ unsigned uniform_(unsigned x) { return __reduce_or_sync(0xffffffffu, x); }
 __device__ __forceinline__ int uniform_(int x) { return (int)uniform_((unsigned)x); }
 __device__ __forceinline__ float uniform_(float x) { return __uint_as_float(uniform_(__float_as_uint(x))); }
@@ -172,7 +174,8 @@ __global__ void __launch_bounds__(32 * kQuadWarps, 1) k_flight_quad(FlightArgs a
     const int n_work = uniform_(a.active_in ? *a.n_active_in : a.n_flights);
     const int end = min(a.step_end, a.max_steps);
 
-    int flight = -1, step = 0;  // of this lane's slot
+    WindLane wl = wind_lane(lane, 0.0f);  // of this lane's slot, as
+    int flight = -1, step = 0;
     unsigned deck2 = 0;         // slots whose plane has pairs in shared memory (warp-uniform)
     unsigned busy = 0;          // slots in flight (warp-uniform)
     bool more = true;
@@ -206,7 +209,7 @@ __global__ void __launch_bounds__(32 * kQuadWarps, 1) k_flight_quad(FlightArgs a
                 release(sc, pmp, cg, &nst.st);
             else
                 nst.st = a.state[fl];
-            if (g == slot) { flight = fl; step = nst.st.step; }
+            if (g == slot) { flight = fl; step = nst.st.step; wl = wind_lane(lane, nfc.fc.phase); }
             if (lane == 0) {
 #pragma unroll
                 for (int i = 0; i < 6; i++) sf[slot].fc[i] = nfc.v[i];
@@ -258,7 +261,7 @@ __global__ void __launch_bounds__(32 * kQuadWarps, 1) k_flight_quad(FlightArgs a
                 for (int i = 0; i < 6; i++) cw.v[i] = sf[g].fc[i];
 #pragma unroll
                 for (int i = 0; i < 4; i++) sw.v[i] = sf[g].st[i];
-                const StepPre pre = fast_pre(cw.fc, sw.st, step);
+                const StepPre pre = fast_pre<true>(cw.fc, sw.st, step, &wl);
                 __syncwarp();  // the last step's reads of k are done
                 if ((lane & 7) == 0) {
                     float4* k = sf[g].k;
@@ -274,10 +277,10 @@ __global__ void __launch_bounds__(32 * kQuadWarps, 1) k_flight_quad(FlightArgs a
             __syncwarp();
             float sum[6];
             // slots 0 and 2, folded over lane bit 4, then 1 and 3; the two results over lane bit 3
-#pragma unroll 1
+#pragma unroll
             for (int half = 0; half < 2; half++) {
                 float u[6];
-#pragma unroll 1
+#pragma unroll
                 for (int part = 0; part < 2; part++) {
                     const int slot = half + 2 * part;
                     float v[6] = {0, 0, 0, 0, 0, 0};
@@ -293,7 +296,7 @@ __global__ void __launch_bounds__(32 * kQuadWarps, 1) k_flight_quad(FlightArgs a
                         k.wbx = bcu(ux); k.wby = bcu(uy); k.wbz = bcu(uz);
                         k.nwbx = bcu(ux ^ 0x80000000u); k.nwby = bcu(uy ^ 0x80000000u); k.nwbz = bcu(uz ^ 0x80000000u);
                         k.cf = bcu(ucf);
-                        k.k19 = bc(PE_CN_SLOPE); k.tiny = bc(1e-30f); k.mone = bc(-1.0f);
+                        k.k19 = c_k19; k.tiny = c_tiny; k.mone = c_mone;
                         const int at = tm_first + slot;
                         TmWords x;
                         tm_load(tm + kTmCol32 + 32 * at, tm + kTmCol8 + 8 * at, tm + kTmCol2 + 2 * at, x);

@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(32 * kWideWarps, 4) k_flight_wide(FlightArgs a
                 k.vbx = bc(vb.x); k.vby = bc(vb.y); k.vbz = bc(vb.z);
                 k.wbx = pk(u0.x, u0.y); k.wby = pk(u0.z, u0.w); k.wbz = pk(u1.x, u1.y);
                 k.nwbx = pk(u1.z, u1.w); k.nwby = pk(u2.x, u2.y); k.nwbz = pk(u2.z, u2.w);
-                k.k19 = bc(PE_CN_SLOPE); k.cf = bc(fc.skin_cf); k.tiny = bc(1e-30f); k.mone = bc(-1.0f);
+                k.k19 = c_k19; k.cf = bc(fc.skin_cf); k.tiny = c_tiny; k.mone = c_mone;
                 f2 nx, ny, nz;
                 pair_force(q0.rbx, q0.rby, q0.rbz, q0.ak, q0.nbx, q0.nby, q0.nbz, k, fc.skin_cf, nx, ny, nz);
                 sm.nf[w][0][lane] = nx; sm.nf[w][1][lane] = ny; sm.nf[w][2][lane] = nz;

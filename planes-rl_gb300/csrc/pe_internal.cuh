@@ -111,7 +111,7 @@ cudaError_t launch_flight_fast(const FlightArgs& a, const FlightShape& sh, int g
 //   32 lanes, hand-over    0.82   1.02   1.39   1.76   2.32   3.92      -
 //   four per warp, same    0.87   1.21   1.50     -    2.08   3.36   10.8
 // Hand-over at 2, 4, 8 and 12 flights per SM: 2.22, 2.07, 2.06, 2.10 ms at 54; none: 2.74.
-constexpr long long kWideFlights = 8;    // per SM: at most this many take a block each
+constexpr long long kWideFlights = 6;    // per SM: at most this many take a block each
 constexpr long long kLanesFlights = 32;  // at most this many 32 lanes each, more four per warp
 constexpr int kHandOver = 6;             // the last flights per SM go on with a block each
 constexpr long long kGradLanesFlights = 192;
