@@ -48,3 +48,17 @@ def test_audit_100k_scenarios(cuda, pe, engine, oracle, host_golden):
     np.testing.assert_array_equal(out2["stats"], out["stats"])
     print("audit of 100,000 scenarios on the device: %.1f ms; %s" %
           (dt * 1e3, dict(zip(pe.AUDIT_NAMES, np.round(out["stats"], 3).tolist()))))
+
+
+@pytest.mark.parametrize("n", [1023, 1024, 1025, 4096, 8191, 8192, 8193, 16385, 70001])
+def test_distance_stats_at_the_edges_of_blocks_and_tiles(cuda, pe, oracle, n):
+    """About the sort's blocks (8192 keys) and the sums' tiles (1024 terms), with ties, all failures and none."""
+    torch = cuda
+    rng = np.random.default_rng(n)
+    for shift in (5.0, -50.0, 500.0):
+        d = (rng.normal(shift, 3, n)).astype(np.float32)
+        d[::7] = d[0]
+        st = torch.empty(13, device="cuda")
+        pe.distance_stats(torch.from_numpy(d).cuda(), n, st)
+        torch.cuda.synchronize()
+        assert np.array_equal(st.cpu().numpy().view(np.uint32), oracle.audit_stats(d).view(np.uint32)), shift
