@@ -333,9 +333,8 @@ cudaError_t record_event(cudaEvent_t ev, cudaStream_t s) {
 int enqueue_eval(pe_engine* e, const float* d_genomes, int pop, int nseeds, int vary, int max_steps,
                  float* dist, int* steps, float* scores, cudaStream_t s, int* launches) {
     PE_CUDA(record_event(e->ev[0], s));
-    launch_prepare(prep_args(e, d_genomes, pop), e->total.p, s);
+    *launches += launch_prepare(prep_args(e, d_genomes, pop), e->total.p, s);
     PE_CUDA(cudaGetLastError());
-    *launches += 3;
     PE_CUDA(record_event(e->ev[1], s));
     int rc = enqueue_fly(e, pop, nseeds, vary, max_steps, dist, steps, s, launches);
     if (rc != PE_OK) return rc;
@@ -604,7 +603,7 @@ int pe_grad(pe_engine* e, const float* d_genomes, int pop, const int* h_seeds, i
     a.obj = d_obj;
     a.grad = d_grad;
     PE_CUDA(record_event(e->ev[0], s));
-    launch_prepare(prep_args(e, d_genomes, pop), e->total.p, s);
+    const int prepare = launch_prepare(prep_args(e, d_genomes, pop), e->total.p, s);
     PE_CUDA(cudaGetLastError());
     PE_CUDA(record_event(e->ev[1], s));
     // the forward pass: the evaluation's body-frame kernel on the model's set-up records, smoothed
@@ -672,9 +671,9 @@ int pe_grad(pe_engine* e, const float* d_genomes, int pop, const int* h_seeds, i
     }
     PE_CUDA(launch_grad(a, fa, e->nsm, e->g_fwd_bps, e->wide_bps, e->g_rev_grid, s, e->ev[2]));
     PE_CUDA(record_event(e->ev[3], s));
-    // prepare (3), set-up, forward (two kernels with the hand-over), order, reverse (five kernels parallel
+    // prepare, set-up, forward (two kernels with the hand-over), order, reverse (five kernels parallel
     // in time, two with the pipelined pass), weights, genome
-    e->last_launches = 3 + 6 + (hand_over && nf > kWideFlights * e->nsm ? 1 : 0) + (a.rec ? 4 + (max_steps > rec_steps) : a.n_long > 0);
+    e->last_launches = prepare + 6 + (hand_over && nf > kWideFlights * e->nsm ? 1 : 0) + (a.rec ? 4 + (max_steps > rec_steps) : a.n_long > 0);
     e->prepared_pop = pop;
     e->timed = true;
     return PE_OK;

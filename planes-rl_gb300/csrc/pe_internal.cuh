@@ -31,7 +31,7 @@ struct PrepArgs {
 
 constexpr int kScanBlock = 1024;  // genomes per block of the prefix scan
 
-void launch_prepare(const PrepArgs& a, int* d_total, cudaStream_t s);
+int launch_prepare(const PrepArgs& a, int* d_total, cudaStream_t s);  // returns the kernels launched
 // Parity probe: 1 = correctly rounded chordwise stations (default), 0 = run-time quotient.
 cudaError_t set_station_mode(int ieee);
 

@@ -306,10 +306,11 @@ struct MassProps {
 };
 
 // src/common.h:311-365 by one warp.  The lanes compute every triangle's terms in parallel into
-// shared memory (T: kMpTerms x kNtMax floats, term k of triangle i at T[k * kNtMax + i]); lane 0
-// then adds them in emission order with the same expressions as a one-thread loop, so the sums
-// round exactly as the reference's serial loop does.  Two passes, as in the reference: the centre
-// of mass first, then the inertia about it.  The 3x3 inverse that the flight never reads (the
+// shared memory (T: kMpTerms x kNtMax floats, term k of triangle i at T[k * kNtMax + i]); then each
+// sum is one lane's, added in emission order with the multiply-adds of a one-thread loop, so the sums
+// round exactly as the reference's serial loop does.  (All on lane 0, the chains shared its issue
+// slots: 17.1 us a plane alone and 207 us for 8,192, now 14.2 and 174.)  Two passes, as
+// in the reference: the centre of mass first, then the inertia about it.  The 3x3 inverse that the flight never reads (the
 // print-varied inverse replaces it) is taken in FP64.  Called by all 32 lanes; *mp on lane 0.
 constexpr int kMpTerms = 15;
 static __device__ __noinline__ void mass_props(GenomeRef g, const vec3* V, const Topo& tp, int lane, float* T,
@@ -323,14 +324,20 @@ static __device__ __noinline__ void mass_props(GenomeRef g, const vec3* V, const
         T[i] = mi; T[kNtMax + i] = ct.x; T[2 * kNtMax + i] = ct.y; T[3 * kNtMax + i] = ct.z;
     }
     __syncwarp();
-    float m = 0, mn = 0;
-    vec3 c = mk3(0, 0, 0), np = mk3(0, 0, 0);
+    // lane 0 the mass, lanes 1..3 the mass moments: a chain of one multiply-add per triangle each
+    const float* tc = T + min(lane, 3) * kNtMax;
+    float sum = 0;
     if (lane == 0) {
-        for (int i = 0; i < tp.nt; i++) {
-            float mi = T[i];
-            vec3 ct = mk3(T[kNtMax + i], T[2 * kNtMax + i], T[3 * kNtMax + i]);
-            m += mi; c = vadd(c, vscl(ct, mi));
-        }
+#pragma unroll 8
+        for (int i = 0; i < tp.nt; i++) sum += T[i];
+    } else {
+#pragma unroll 8
+        for (int i = 0; i < tp.nt; i++) sum = fmaf(tc[i], T[i], sum);
+    }
+    float m = __shfl_sync(0xffffffffu, sum, 0), mn = 0;
+    vec3 c = mk3(__shfl_sync(0xffffffffu, sum, 1), __shfl_sync(0xffffffffu, sum, 2), __shfl_sync(0xffffffffu, sum, 3));
+    vec3 np = mk3(0, 0, 0);
+    if (lane == 0) {
         float shell_m = m;
         np = mk3(0.5f * g[G_CHORD], 0, 0);
         mn = g[G_NOSE] * shell_m;
@@ -365,18 +372,22 @@ static __device__ __noinline__ void mass_props(GenomeRef g, const vec3* V, const
         t[13 * kNtMax] = nn.y; t[14 * kNtMax] = nn.z;
     }
     __syncwarp();
-    if (lane != 0) return;
-    float I[6] = {0, 0, 0, 0, 0, 0};
+    // lane k the component I[k]: two multiply-adds per triangle, xx yy zz adding and xy xz yz subtracting
+    const int k = min(lane, 5);
+    const float* t1 = T + (1 + k) * kNtMax;                      // mi *
+    const float* t2 = T + (k < 3 ? 7 : (k < 5 ? 11 : 12)) * kNtMax;  // then this
+    const float* t3 = T + (k < 3 ? 8 + k : (k == 3 ? 13 : 14)) * kNtMax;  // times this
+    const float sign = k < 3 ? 1.0f : -1.0f;
+    float part = 0;
+#pragma unroll 4
     for (int i = 0; i < tp.nt; i++) {
-        const float* t = T + i;
-        float mi = t[0];
-        I[0] += mi * t[kNtMax]; I[1] += mi * t[2 * kNtMax]; I[2] += mi * t[3 * kNtMax];
-        I[3] -= mi * t[4 * kNtMax]; I[4] -= mi * t[5 * kNtMax]; I[5] -= mi * t[6 * kNtMax];
-        float th = t[7 * kNtMax];
-        I[0] += th * t[8 * kNtMax]; I[1] += th * t[9 * kNtMax]; I[2] += th * t[10 * kNtMax];
-        I[3] -= t[11 * kNtMax] * t[13 * kNtMax]; I[4] -= t[11 * kNtMax] * t[14 * kNtMax];
-        I[5] -= t[12 * kNtMax] * t[14 * kNtMax];
+        part = fmaf(sign * T[i], t1[i], part);
+        part = fmaf(sign * t2[i], t3[i], part);
     }
+    float I[6];
+#pragma unroll
+    for (int q = 0; q < 6; q++) I[q] = __shfl_sync(0xffffffffu, part, q);
+    if (lane != 0) return;
     {
         vec3 r = vsub(np, c);
         I[0] += mn * (r.y * r.y + r.z * r.z); I[1] += mn * (r.x * r.x + r.z * r.z);

@@ -1,21 +1,20 @@
 // pe_prepare.cu -- genome -> mesh -> mass properties -> packed panels (src/sim.cu:25-49).
 //
-// Three launches:
+// Three launches, two for at most kScanBlock genomes:
 //   k_topo_scan   triangle count of each genome from its topology genes alone, block-local
 //                 exclusive scan, block totals out.
 //   k_scan_tot    exclusive scan of the block totals (one block, 1024 at a time); also the
 //                 grand total.
 //   k_mesh        one warp per plane: lanes evaluate the mesh vertices in parallel into shared
-//                 memory and every triangle's mass-property terms likewise; lane 0 adds the terms
-//                 in emission order (the reference's order, so the sums round identically); lanes
-//                 write the COM-relative panel SoA into the plane's exact prefix range.
-// HBM traffic is small (140 B genome in, 32 B per panel out); the cost is lane 0's ordered
-// additions, about 1 ms per 100k planes.
+//                 memory and every triangle's mass-property terms likewise; then each sum is one
+//                 lane's, in emission order (the reference's order, so the sums round identically);
+//                 lanes write the COM-relative panel SoA into the plane's exact prefix range.
+// HBM traffic is small (140 B genome in, 32 B per panel out); the cost is the ordered sums.
 #include "pe_internal.cuh"
 
 namespace pe {
 
-__global__ void __launch_bounds__(kScanBlock) k_topo_scan(PrepArgs a) {
+__global__ void __launch_bounds__(kScanBlock) k_topo_scan(PrepArgs a, int* total) {
     __shared__ int warp_tot[kScanBlock / 32];
     int p = blockIdx.x * kScanBlock + threadIdx.x;
     int n = 0;
@@ -43,7 +42,10 @@ __global__ void __launch_bounds__(kScanBlock) k_topo_scan(PrepArgs a) {
     __syncthreads();
     int excl = x - n + (w > 0 ? warp_tot[w - 1] : 0);
     if (p < a.pop) a.pt.off[p] = excl;  // block-local for now
-    if (threadIdx.x == kScanBlock - 1) a.block_sum[blockIdx.x] = excl + n;
+    if (threadIdx.x == kScanBlock - 1) {
+        a.block_sum[blockIdx.x] = gridDim.x == 1 ? 0 : excl + n;
+        if (gridDim.x == 1) *total = excl + n;  // one block's totals need no scan of their own
+    }
 }
 
 // Exclusive scan of nblocks block totals in place, in tiles of 1024 with the running sum of the
@@ -155,11 +157,12 @@ cudaError_t set_station_mode(int ieee) {
     return cudaMemcpyToSymbol(c_station_ieee, &v, sizeof(int));
 }
 
-void launch_prepare(const PrepArgs& a, int* d_total, cudaStream_t s) {
+int launch_prepare(const PrepArgs& a, int* d_total, cudaStream_t s) {
     int nb = (a.pop + kScanBlock - 1) / kScanBlock;
-    k_topo_scan<<<nb, kScanBlock, 0, s>>>(a);
-    k_scan_tot<<<1, 1024, 0, s>>>(a.block_sum, nb, d_total);
+    k_topo_scan<<<nb, kScanBlock, 0, s>>>(a, d_total);
+    if (nb > 1) k_scan_tot<<<1, 1024, 0, s>>>(a.block_sum, nb, d_total);
     k_mesh<<<(a.pop + kMeshWarps - 1) / kMeshWarps, kMeshWarps * 32, 0, s>>>(a);
+    return nb > 1 ? 3 : 2;
 }
 
 }  // namespace pe
