@@ -11,6 +11,7 @@
 //                   the triangles with block reductions) and panels, in T.
 //   k_obj_forward   one block of kObjW warps per flight, persistent over a work queue: print
 //                   variation, staging, release and the flight; writes the smoothed distance.
+//   k_obj_forward4  the same with four flights per block, for many flights and for FP64.
 //   k_obj_weights   one block per plane: the tail-aware objective of its distances.
 #include <cuda_runtime.h>
 
@@ -212,6 +213,168 @@ __global__ void __launch_bounds__(32 * kObjW) k_obj_forward(ObjArgs a) {
     }
 }
 
+// One of a block's four flights, and the warp's of the same number.
+template <class T>
+struct ObjSlot {
+    T part[kObjW][8];  // each warp's sums of the step's force and torque
+    T pre[8];          // vb xyz, w xyz, skin friction
+    T sp[7 * kNtMax];  // staged panels (SoA)
+};
+
+// The sums over a warp of 24 values per lane (six of each of four flights), transposed: a level halves
+// the values a lane carries, 24 shuffles instead of 120, and each sum follows the xor tree that a
+// butterfly over all lanes would.  Lane 8 m + 4 h + q (q < 3) returns component 3 h + q of flight m.
+template <class T>
+__device__ __forceinline__ T warp_sum24(T (&v)[24], int lane) {
+    auto fold = [&](int m, int half) {
+        const bool up = (lane & m) != 0;
+#pragma unroll
+        for (int i = 0; i < half; i++) {
+            const T send = up ? v[i] : v[i + half];
+            const T keep = up ? v[i + half] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, m);
+        }
+    };
+    fold(16, 12);
+    fold(8, 6);
+    fold(4, 3);
+    v[3] = T(0);
+    fold(2, 2);
+    fold(1, 1);
+    return v[0];
+}
+
+// Four flights per block: all warps take the panels of every flight, each warp its own flight's integrator
+// and gusts, so a flight-step is 1,100 warp instructions instead of 3,000 and twenty flights fill an SM
+// instead of five (FP32).  Two barriers per step and a longer chain: for batches of many flights.
+template <class T>
+__global__ void __launch_bounds__(32 * kObjW, 1) k_obj_forward4(ObjArgs a) {
+    using V3T = pg::V3<T>;
+    constexpr int nthr = 32 * kObjW;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    ObjSlot<T>* slot = reinterpret_cast<ObjSlot<T>*>(smem_raw);
+    __shared__ int s_nt[kObjW];  // panels of each slot's flight (0: none)
+    static_assert(kObjW == 4, "warp_sum24 takes four flights");
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int n_flights = a.pop * a.nseeds;
+    ObjSlot<T>& mine = slot[warp];
+    int f = 0, j = 0, to_chunk = 0;
+    bool live = false;
+    pg::FlightP<T> P;
+    pg::St<T> s;
+    pg::Pre<T> pr{};
+    auto publish = [&]() {
+        if (lane == 0) {
+            mine.pre[0] = pr.vb.x; mine.pre[1] = pr.vb.y; mine.pre[2] = pr.vb.z;
+            mine.pre[3] = pr.w.x; mine.pre[4] = pr.w.y; mine.pre[5] = pr.w.z;
+        }
+    };
+    auto next_flight = [&]() {
+        for (;;) {
+            if (lane == 0) f = atomicAdd(a.work, 1);
+            f = __shfl_sync(0xffffffffu, f, 0);
+            live = f < n_flights;
+            if (!live) {
+                if (lane == 0) s_nt[warp] = 0;
+                return;
+            }
+            const int p = f / a.nseeds, si = f - p * a.nseeds;
+            const T* pl = reinterpret_cast<const T*>(a.plane) + (size_t)p * kObjPlaneStride;
+            const int nt = (int)pl[7];
+            if (nt <= 0) {  // does not fit the print volume
+                if (lane == 0) a.dist[f] = -100.0;
+                continue;
+            }
+            const int seed = a.seeds[si] + (a.vary ? p * 7919 : 0);
+            Scenario S;
+            scenario_desc(seed, &S);
+            T sc[kScenN];
+#pragma unroll
+            for (int k = 0; k < kScenN; k++) sc[k] = (T)S.v[k];
+            V3T cg;
+            T sigma, beta[6], I[6];
+#pragma unroll
+            for (int q = 0; q < 6; q++) I[q] = pl[1 + q];
+            pg::printed(sc, pl[0], I, P, &cg, &sigma, beta);
+            P.phase = (T)seed_phase(seed);
+            const T* pc = pl + 8;
+            T* sp = mine.sp;
+            for (int i = lane; i < nt; i += 32) {
+                V3T rb, nb;
+                T ak;
+                pg::stage(pg::v3(pc[i], pc[kNtMax + i], pc[2 * kNtMax + i]), pc[3 * kNtMax + i],
+                          pg::v3(pc[4 * kNtMax + i], pc[5 * kNtMax + i], pc[6 * kNtMax + i]), cg, sc[pg::SC_RHO],
+                          sc[pg::SC_WP], sc[pg::SC_WR], &rb, &nb, &ak);
+                sp[i] = rb.x; sp[kNtMax + i] = rb.y; sp[2 * kNtMax + i] = rb.z;
+                sp[3 * kNtMax + i] = nb.x; sp[4 * kNtMax + i] = nb.y; sp[5 * kNtMax + i] = nb.z;
+                sp[6 * kNtMax + i] = ak;
+            }
+            s = pg::release(sc, P, cg, (V3T*)nullptr, (V3T*)nullptr);
+            pg::step_pre(P, s, pr);
+            publish();
+            if (lane == 0) {
+                mine.pre[6] = P.cf;
+                s_nt[warp] = nt;
+            }
+            j = 0;
+            to_chunk = kChunk;
+            return;
+        }
+    };
+    next_flight();
+    for (;;) {
+        __syncthreads();
+        if (!(s_nt[0] | s_nt[1] | s_nt[2] | s_nt[3])) break;
+        T v[24];
+#pragma unroll
+        for (int m = 0; m < kObjW; m++) {
+            T acc[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
+            const T* pre = slot[m].pre;
+            pg::Pre<T> q;
+            q.vb = pg::v3(pre[0], pre[1], pre[2]);
+            q.w = pg::v3(pre[3], pre[4], pre[5]);
+            const int nt = s_nt[m];
+            const T* sp = slot[m].sp;
+            const T cf = pre[6];
+            for (int i = tid; i < nt; i += nthr) {
+                V3T fo, tq;
+                pg::panel_fwd(q, pg::v3(sp[i], sp[kNtMax + i], sp[2 * kNtMax + i]),
+                              pg::v3(sp[3 * kNtMax + i], sp[4 * kNtMax + i], sp[5 * kNtMax + i]), sp[6 * kNtMax + i],
+                              cf, &fo, &tq);
+                acc[0] += fo.x; acc[1] += fo.y; acc[2] += fo.z;
+                acc[3] += tq.x; acc[4] += tq.y; acc[5] += tq.z;
+            }
+#pragma unroll
+            for (int k = 0; k < 6; k++) v[6 * m + k] = acc[k];
+        }
+        const T total = warp_sum24(v, lane);
+        if ((lane & 3) != 3) slot[lane >> 3].part[warp][3 * ((lane >> 2) & 1) + (lane & 3)] = total;
+        __syncthreads();
+        if (!live) continue;
+        T w[6];
+#pragma unroll
+        for (int k = 0; k < 6; k++) {
+            T t = mine.part[0][k];
+#pragma unroll
+            for (int q = 1; q < kObjW; q++) t += mine.part[q][k];
+            w[k] = t;
+        }
+        const pg::St<T> nx = pg::step_post(P, s, pr, pg::v3(w[0], w[1], w[2]), pg::v3(w[3], w[4], w[5]));
+        T d = T(0);
+        int kind = 0;
+        if (pg::terminate(s, nx, j, a.max_steps, &d, &kind)) {
+            if (lane == 0) a.dist[f] = (double)d;
+            next_flight();
+        } else {
+            s = nx;
+            if (--to_chunk == 0) { s.t = T((double)(j + 1)) * T(pg::kDt); to_chunk = kChunk; }  // src/sim.cu:113
+            j++;
+            pg::step_pre(P, s, pr);
+            publish();
+        }
+    }
+}
+
 template <class T>
 __global__ void __launch_bounds__(32) k_obj_weights(ObjArgs a) {
     __shared__ T d[kGradMaxSeeds], w[kGradMaxSeeds];
@@ -228,16 +391,23 @@ size_t forward_smem() {
 
 template <class T>
 cudaError_t launch_t(const ObjArgs& a, int nsm, cudaStream_t s) {
-    cudaError_t e = cudaFuncSetAttribute(k_obj_forward<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)forward_smem<T>());
+    // Measured with a flight / four flights per block, FP32: 1.81 / 1.99 ms at 256 x 8, 2.47 / 2.28 at
+    // 384 x 8, 3.19 / 2.57 at 512 x 8, 7.76 / 5.55 at 1500 x 8; FP64: 17.1 / 17.1 at 16 x 2, 37.5 / 34.4 at
+    // 64 x 8, 162 / 93 at 512 x 8.
+    const bool four = sizeof(T) == 8 || (long long)a.pop * a.nseeds > 16LL * nsm;
+    const void* fn = four ? (const void*)k_obj_forward4<T> : (const void*)k_obj_forward<T>;
+    const size_t smem = four ? kObjW * sizeof(ObjSlot<T>) : forward_smem<T>();
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int bpsm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, k_obj_forward<T>, 32 * kObjW, forward_smem<T>());
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, fn, 32 * kObjW, smem);
     if (e != cudaSuccess) return e;
     e = cudaMemsetAsync(a.work, 0, sizeof(int), s);
     if (e != cudaSuccess) return e;
+    const int grid = (bpsm > 0 ? bpsm : 1) * nsm;
     k_obj_prepare<T><<<a.pop, kObjThreads, 0, s>>>(a);
-    k_obj_forward<T><<<(bpsm > 0 ? bpsm : 1) * nsm, 32 * kObjW, forward_smem<T>(), s>>>(a);
+    if (four) k_obj_forward4<T><<<grid, 32 * kObjW, smem, s>>>(a);
+    else k_obj_forward<T><<<grid, 32 * kObjW, smem, s>>>(a);
     if (a.obj) k_obj_weights<T><<<a.pop, 32, 0, s>>>(a);
     return cudaGetLastError();
 }

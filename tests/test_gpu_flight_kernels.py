@@ -107,3 +107,28 @@ def test_gradient_parallel_in_time(cuda, pe, oracle, monkeypatch, pop, nseeds, m
     assert np.array_equal(np.isnan(a[2]), np.isnan(b[2])) and bad.sum() <= 1
     norm = np.linalg.norm(b[2][~bad], axis=1)
     assert (np.linalg.norm((a[2] - b[2])[~bad], axis=1) <= 1e-5 * norm).all()
+
+
+@pytest.mark.parametrize("max_steps", [1, 2, 600, 601, 900])
+def test_objective_flights_per_block(cuda, pe, oracle, max_steps):
+    """pe_objective with a flight per block (few flights, FP32) and with four (many flights): the same
+    distances bit for bit, and FP64 (four per block) within FP32's rounding of them for flights this short
+    of chaos (1e-3 of a metre for 99 % of flights; the rest pass through the FP32 gust sine's worst arguments)."""
+    torch = cuda
+    sm = torch.cuda.get_device_properties(0).multi_processor_count
+    pop = 16 * sm // 7 + 3  # 7 scenarios: just over 16 flights per SM
+    G, seeds = oracle.grand(51, pop), list(range(2, 9))
+    e = pe.Engine(0)
+
+    def dist(g, precision):
+        n = g.shape[0]
+        obj, d = (torch.empty(k, dtype=torch.float64, device="cuda") for k in (n, 7 * n))
+        e.objective(torch.from_numpy(g).cuda(), n, seeds, precision=precision, max_steps=max_steps, d_obj=obj, d_dist=d)
+        torch.cuda.synchronize()
+        return obj.cpu().numpy(), d.cpu().numpy()
+
+    many, few = dist(G, 32), dist(np.ascontiguousarray(G[5:45]), 32)
+    assert np.array_equal(many[1][35:315], few[1]) and np.array_equal(many[0][5:45], few[0])
+    wide = dist(G, 64)
+    assert np.mean(np.abs(wide[1] - many[1]) <= 1e-3) >= 0.99
+    e.close()
