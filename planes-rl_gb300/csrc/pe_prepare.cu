@@ -1,6 +1,6 @@
 // pe_prepare.cu -- genome -> mesh -> mass properties -> packed panels (src/sim.cu:25-49).
 //
-// Three launches, two for at most kScanBlock genomes:
+// Three launches, two for at most kScanAlone genomes:
 //   k_topo_scan   triangle count of each genome from its topology genes alone, block-local
 //                 exclusive scan, block totals out.
 //   k_scan_tot    exclusive scan of the block totals (one block, 1024 at a time); also the
@@ -43,8 +43,8 @@ __global__ void __launch_bounds__(kScanBlock) k_topo_scan(PrepArgs a, int* total
     int excl = x - n + (w > 0 ? warp_tot[w - 1] : 0);
     if (p < a.pop) a.pt.off[p] = excl;  // block-local for now
     if (threadIdx.x == kScanBlock - 1) {
-        a.block_sum[blockIdx.x] = gridDim.x == 1 ? 0 : excl + n;
-        if (gridDim.x == 1) *total = excl + n;  // one block's totals need no scan of their own
+        a.block_sum[blockIdx.x] = total ? 0 : excl + n;
+        if (total) *total = excl + n;  // the only block: its totals need no scan of their own
     }
 }
 
@@ -157,12 +157,18 @@ cudaError_t set_station_mode(int ieee) {
     return cudaMemcpyToSymbol(c_station_ieee, &v, sizeof(int));
 }
 
+// A small batch's preparation is its launches: without the scan's, 2 of 17 us at one genome; from some
+// hundreds on k_mesh and the flights hide it.
+constexpr int kScanAlone = 128;
+static_assert(kScanAlone <= kScanBlock, "one block counts them");
+
 int launch_prepare(const PrepArgs& a, int* d_total, cudaStream_t s) {
     int nb = (a.pop + kScanBlock - 1) / kScanBlock;
-    k_topo_scan<<<nb, kScanBlock, 0, s>>>(a, d_total);
-    if (nb > 1) k_scan_tot<<<1, 1024, 0, s>>>(a.block_sum, nb, d_total);
+    const bool alone = a.pop <= kScanAlone;
+    k_topo_scan<<<nb, kScanBlock, 0, s>>>(a, alone ? d_total : nullptr);
+    if (!alone) k_scan_tot<<<1, 1024, 0, s>>>(a.block_sum, nb, d_total);
     k_mesh<<<(a.pop + kMeshWarps - 1) / kMeshWarps, kMeshWarps * 32, 0, s>>>(a);
-    return nb > 1 ? 3 : 2;
+    return alone ? 2 : 3;
 }
 
 }  // namespace pe
