@@ -91,7 +91,7 @@ typedef struct pe_engine pe_engine;
  * Default: lanes 16, warps 1, chunk 7200, blocks 0, use_graph 0, formulation 1, reg_cap 3. */
 typedef struct {
     int lanes;       /* lanes per flight: 16 or 32 (formulation 0: 32 only) */
-    int warps;       /* warps per block of the flight kernel: 1..8 */
+    int warps;       /* warps per block of the flight kernel: 1..8 (formulation 0: always 4) */
     int chunk;       /* steps per flight launch: 1..7200 */
     int blocks;      /* flight grid size; 0 = fill the GPU (persistent) */
     int use_graph;   /* 1 = replay the whole evaluation from a captured CUDA graph */

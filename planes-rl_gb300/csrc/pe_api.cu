@@ -204,7 +204,7 @@ int blocks_for(pe_engine* e, const pe_config& c) {
     int& bps = e->bps_cache[c.formulation][c.reg_cap][c.lanes == 16 ? 0 : 1][c.warps];
     if (bps == 0) {
         FlightShape sh{c.lanes, c.warps, c.chunk, 0, c.formulation, c.reg_cap};
-        bps = c.formulation ? flight_fast_blocks_per_sm(sh) : flight_blocks_per_sm(sh);
+        bps = c.formulation ? flight_fast_blocks_per_sm(sh) : flight_blocks_per_sm();
         if (bps <= 0) bps = 1;
     }
     return bps * e->nsm;
@@ -314,7 +314,7 @@ int enqueue_fly(pe_engine* e, int pop, int nseeds, int vary, int max_steps, floa
         a.active_out = k == nchunks - 1 ? nullptr : (k % 2 == 0 ? e->list0.p : e->list1.p);
         a.n_active_out = &nact[k + 1];
         a.work = &work[k];
-        PE_CUDA(c.formulation ? launch_flight_fast(a, sh, grid, s) : launch_flight(a, sh, grid, s));
+        PE_CUDA(c.formulation ? launch_flight_fast(a, sh, grid, s) : launch_flight(a, grid, s));
         (*launches)++;
     }
     return PE_OK;
@@ -853,7 +853,7 @@ int pe_debug_step(pe_engine* e, int pop, const int* h_seeds, int nseeds, int var
                                        d_fit, step, lanes, s));
     else
         PE_CUDA(launch_debug_step(a, (const FlightState*)d_state_in, (FlightState*)d_state_out, d_FT, d_done, d_fit,
-                                  step, lanes, s));
+                                  step, s));
     return PE_OK;
 }
 

@@ -99,9 +99,9 @@ struct FlightShape {
                       // 3 = 184 in one-warp blocks
 };
 
-int flight_blocks_per_sm(const FlightShape& sh);
-size_t flight_smem_bytes(const FlightShape& sh);
-cudaError_t launch_flight(const FlightArgs& a, const FlightShape& sh, int grid, cudaStream_t s);
+// The reference arithmetic (pe_flight.cu): up to four flights per 4-warp block, whatever lanes and warps say.
+int flight_blocks_per_sm();
+cudaError_t launch_flight(const FlightArgs& a, int grid, cudaStream_t s);
 int flight_fast_blocks_per_sm(const FlightShape& sh);
 cudaError_t launch_flight_fast(const FlightArgs& a, const FlightShape& sh, int grid, cudaStream_t s);
 // Which kernels fly a batch in the default shape (results do not depend on it), by flights per SM.
@@ -146,7 +146,7 @@ cudaError_t launch_scores(const float* dist, int pop, int nseeds, float* scores,
 // included) at step `step`, applies one step and writes state_out[f] and FT[f*6..] (aerodynamic
 // force and torque sums, world frame).
 cudaError_t launch_debug_step(const FlightArgs& a, const FlightState* state_in, FlightState* state_out,
-                              float* FT, int* done, float* fit, int step, int lanes, cudaStream_t s);
+                              float* FT, int* done, float* fit, int step, cudaStream_t s);
 
 // Release state of every flight (parity tests).
 cudaError_t launch_debug_release(const FlightArgs& a, FlightState* out, cudaStream_t s);

@@ -132,3 +132,32 @@ def test_objective_flights_per_block(cuda, pe, oracle, max_steps):
     wide = dist(G, 64)
     assert np.mean(np.abs(wide[1] - many[1]) <= 1e-3) >= 0.99
     e.close()
+
+
+@pytest.mark.parametrize("pop,S,max_steps,chunk", [(1, 1, 7200, 7200), (7, 3, 1, 1), (40, 19, 601, 600), (40, 20, 1200, 599),
+                                                   (200, 16, 7200, 600), (800, 16, 7200, 7200)])
+def test_reference_order_blocks(cuda, pe, oracle, pop, S, max_steps, chunk):
+    """The reference arithmetic with one to four flights per block (by the number of flights), in one launch
+    and in chunks: the first planes' flights bit for bit as they fly alone, oversize planes left at -100."""
+    torch = cuda
+    G, seeds = oracle.grand(17, pop), list(range(4, 4 + S))
+
+    def fly(g, steps_per_launch):
+        e = pe.Engine(0)
+        e.set_config(formulation=0, lanes=32, reg_cap=0, chunk=steps_per_launch)
+        n = g.shape[0] * S
+        d, st = torch.empty(n, device="cuda"), torch.empty(n, dtype=torch.int32, device="cuda")
+        e.eval_batch(torch.from_numpy(g).cuda(), g.shape[0], seeds, 0, max_steps, d, st)
+        torch.cuda.synchronize()
+        nt = torch.empty(g.shape[0], dtype=torch.int32, device="cuda")
+        e.plane_table(g.shape[0], d_nt=nt)
+        torch.cuda.synchronize()
+        e.close()
+        return d.cpu().numpy(), st.cpu().numpy(), nt.cpu().numpy()
+
+    d, st, nt = fly(G, chunk)
+    over = np.repeat(nt <= 0, S)
+    assert np.all(d[over] == -100.0) and np.all(st[over] == 0) and np.all(st[~over] > 0) and st.max() <= max_steps
+    for p in range(min(pop, 5)):
+        a = fly(G[p:p + 1], 7200)
+        assert np.array_equal(a[0], d[p * S:(p + 1) * S]) and np.array_equal(a[1], st[p * S:(p + 1) * S])
