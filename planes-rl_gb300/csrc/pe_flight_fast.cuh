@@ -405,21 +405,30 @@ __device__ __forceinline__ void fast_rotate(const FastConst& fc, vec3 gyro, vec3
                         fma_(fc.invI[5], tq.z, fma_(fc.invI[4], tq.y, mul_(fc.invI[3], tq.x))),
                         fma_(fc.invI[8], tq.z, fma_(fc.invI[7], tq.y, mul_(fc.invI[6], tq.x))));
     w = mk3(fma_(dw.x, PE_DT, w.x), fma_(dw.y, PE_DT, w.y), fma_(dw.z, PE_DT, w.z));
-    // a squared length safely below the limit's needs no root (a NaN takes the long way)
+    // q += 0.5 dt q (0, w); normalize
+    auto turn = [&](vec3 v) {
+        const float h = mul_(0.5f, PE_DT);
+        const float dqw = -fma_(q.z, v.z, fma_(q.y, v.y, mul_(q.x, v.x)));
+        const float dqx = fma_(q.y, v.z, fma_(-q.z, v.y, mul_(q.w, v.x)));
+        const float dqy = fma_(q.z, v.x, fma_(-q.x, v.z, mul_(q.w, v.y)));
+        const float dqz = fma_(q.x, v.y, fma_(-q.y, v.x, mul_(q.w, v.z)));
+        const quat4 qn = mkq(fma_(h, dqw, q.w), fma_(h, dqx, q.x), fma_(h, dqy, q.y), fma_(h, dqz, q.z));
+        const float il = rsqrtf(fma_(qn.z, qn.z, fma_(qn.y, qn.y, fma_(qn.x, qn.x, mul_(qn.w, qn.w)))));
+        return mkq(mul_(qn.w, il), mul_(qn.x, il), mul_(qn.y, il), mul_(qn.z, il));
+    };
+    quat4 next = turn(w);
+    // A squared length safely below the limit's needs no root (a NaN takes the long way).  Asked after the
+    // attitude, so that the chain does not wait for the branch.
     const float w2 = dot_(w, w);
     if (!(w2 < 22499.f)) {
         const float wl = sqrtf(w2);
-        if (wl > 150.f) { const float k = __fdiv_rn(150.f, wl); w = mk3(mul_(w.x, k), mul_(w.y, k), mul_(w.z, k)); }
+        if (wl > 150.f) {
+            const float k = __fdiv_rn(150.f, wl);
+            w = mk3(mul_(w.x, k), mul_(w.y, k), mul_(w.z, k));
+            next = turn(w);
+        }
     }
-    // q += 0.5 dt q (0, w); normalize
-    const float h = mul_(0.5f, PE_DT);
-    const float dqw = -fma_(q.z, w.z, fma_(q.y, w.y, mul_(q.x, w.x)));
-    const float dqx = fma_(q.y, w.z, fma_(-q.z, w.y, mul_(q.w, w.x)));
-    const float dqy = fma_(q.z, w.x, fma_(-q.x, w.z, mul_(q.w, w.y)));
-    const float dqz = fma_(q.x, w.y, fma_(-q.y, w.x, mul_(q.w, w.z)));
-    const quat4 qn = mkq(fma_(h, dqw, q.w), fma_(h, dqx, q.x), fma_(h, dqy, q.y), fma_(h, dqz, q.z));
-    const float il = rsqrtf(fma_(qn.z, qn.z, fma_(qn.y, qn.y, fma_(qn.x, qn.x, mul_(qn.w, qn.w)))));
-    q = mkq(mul_(qn.w, il), mul_(qn.x, il), mul_(qn.y, il), mul_(qn.z, il));
+    q = next;
 }
 // The integrator's translation from the world-frame aerodynamic force Fs.
 __device__ __forceinline__ void fast_translate(const FastConst& fc, vec3 Fs, vec3& vel, vec3& pos) {
@@ -427,11 +436,17 @@ __device__ __forceinline__ void fast_translate(const FastConst& fc, vec3 Fs, vec
     const float kv = mul_(fc.invmass, PE_DT);
     vel = mk3(fma_(Fs.x, kv, vel.x), fma_(Fs.y, kv, vel.y), fma_(Fs.z, kv, vel.z));
     const float v2 = dot_(vel, vel);
+    const vec3 from = pos;
+    auto move = [&]() { pos = mk3(fma_(vel.x, PE_DT, from.x), fma_(vel.y, PE_DT, from.y), fma_(vel.z, PE_DT, from.z)); };
+    move();
     if (!(v2 < 3599.f)) {
         const float vl = sqrtf(v2);
-        if (vl > 60.f) { const float k = __fdiv_rn(60.f, vl); vel = mk3(mul_(vel.x, k), mul_(vel.y, k), mul_(vel.z, k)); }
+        if (vl > 60.f) {
+            const float k = __fdiv_rn(60.f, vl);
+            vel = mk3(mul_(vel.x, k), mul_(vel.y, k), mul_(vel.z, k));
+            move();
+        }
     }
-    pos = mk3(fma_(vel.x, PE_DT, pos.x), fma_(vel.y, PE_DT, pos.y), fma_(vel.z, PE_DT, pos.z));
 }
 // Whether the flight ends at `step`.
 __device__ __forceinline__ bool fast_over(vec3 pos, vec3 vel, int step, int max_steps) {

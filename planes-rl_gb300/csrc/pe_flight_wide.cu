@@ -6,18 +6,21 @@
 //   * a lane holds its one or two pairs in registers for the whole flight (pass n on warp n % 3), so the
 //     panel part is one pair's chain with no loads;
 //   * the pair forces cross through shared memory, and warp w adds components w of force and torque over
-//     the passes in their fixed order;
-//   * the lane totals cross once more, and the fold takes eight totals per lane (three levels of the tree
-//     without a shuffle) and the last four results at once;
+//     the passes in their fixed order, its own passes from registers;
+//   * the lane totals cross once more, and the fold takes sixteen totals per lane (four levels of the tree
+//     without a shuffle);
 //   * warp 0 turns the plane while warp 1 moves it and takes its gusts, one sine per lane; warp 2 stores
 //     what pe_grad keeps.  Attitude rows, rates and air velocity cross through shared memory.
-// Three barriers of three warps per step; 0.39 us a step alone.  Bound: that chain, and from four
-// flights per SM on the 800 warp instructions of a flight-step, twice the other kernels', so the
-// dispatch gives it small batches and the last flights of large ones (pe_internal.cuh).
+// Three barriers of three warps per step.  The step's code is instantiated for each warp: its own values stay
+// in registers, all lanes store what one would (no branch), the rates cross once and are doubled by the
+// readers.  Bound: that chain, 0.38 us a step alone, a fifth of it shared-memory wavefronts, and from six
+// flights per SM on the 800 warp instructions of a flight-step, twice the other kernels', so the dispatch
+// gives it small batches and the last flights of large ones (pe_internal.cuh).
 // Measured, flights of 64 x 8 (longest 1,368 steps): 0.96 ms at 32 lanes; here 0.84 ms with every warp
 // integrating, 0.76 ms with the integrator split, 0.63 ms with its branches and clamps off the chain and
-// the sines spread.  The sums run in the fixed order of pe_flight_fast.cuh: every distance and step
-// count is bit-identical to the other kernels'.
+// the sines spread, 0.53 ms with the code by warp and the shorter fold.  (Six warps of a pass each: 0.64;
+// the two pairs of a lane overlap.  Five blocks per SM at 128 registers: 0.56.)  The sums run in the fixed
+// order of pe_flight_fast.cuh: every distance and step count is bit-identical to the other kernels'.
 #include <type_traits>
 
 #include "pe_flight_fast.cuh"
@@ -31,10 +34,11 @@ constexpr int kWidePasses = 6;  // pair v + 32 n of pass n: 192 pairs hold the l
 static_assert(32 * kWidePasses >= (kNtMax + 1) / 2, "every pair has a pass");
 
 struct WideSmem {
-    f2 nf[kWidePasses][3][32];  // -force of each pair, packed (even, odd panel)
-    float tot[6][36];           // lane totals of the six sums, lane v at (v % 4) * 8 + v / 4
-    float4 rows[3];             // attitude rows, from warp 0
-    float4 rate[3];             // body rates xyz and their negatives, each twice, from warp 0
+    // -force of each pair, packed (even, odd panel): x and y, z
+    ulonglong2 nf_xy[kWidePasses][32];
+    f2 nf_z[kWidePasses][32];
+    alignas(16) float tot[6][36];           // lane totals of the six sums, lane v at (v % 4) * 8 + v / 4
+    float4 rows[3];             // attitude rows and body rates, from warp 0
     float4 air;                 // air velocity; as an int 1 once the flight is over, 2 at the launch's last step; warp 1
     int next;
 };
@@ -63,32 +67,27 @@ __device__ __forceinline__ WidePair wide_stage(const FlightArgs& a, int off, int
 
 __device__ __forceinline__ f2 axis(f2 x, f2 y, f2 z, int i) { return i == 0 ? x : (i == 1 ? y : z); }
 
-// Three of the six sums on every lane: lanes 4c + r fold the totals of lanes r, r + 4, ..., r + 28 of
-// sum first + c by bits 16, 8 and 4; the last two levels take the four results of a sum at once.
+// Three of the six sums on every lane: lanes 2c + r fold the totals of lanes r and r + 2, r + 4, ... of sum
+// first + c by bits 16, 8, 4 and 2; the last level takes both results of a sum at once.  (Four lanes per sum
+// and twelve shuffles: 3 % more per step; one lane and three: 2 %.)
 __device__ __forceinline__ vec3 wide_fold(const WideSmem& sm, int first, int lane) {
-    const float4* row = reinterpret_cast<const float4*>(&sm.tot[first + min(lane >> 2, 2)][(lane & 3) * 8]);
-    const float4 lo = row[0], hi = row[1];
-    const float t = add_(add_(add_(lo.x, hi.x), add_(lo.z, hi.z)), add_(add_(lo.y, hi.y), add_(lo.w, hi.w)));
+    const ulonglong2* row = reinterpret_cast<const ulonglong2*>(&sm.tot[first + min(lane >> 1, 2)][(lane & 1) * 8]);
+    const ulonglong2 lo = row[0], hi = row[1], lo2 = row[4], hi2 = row[5];
+    float t0, t1, u0, u1;
+    upk(add2(add2(lo.x, hi.x), add2(lo.y, hi.y)), t0, t1);
+    upk(add2(add2(lo2.x, hi2.x), add2(lo2.y, hi2.y)), u0, u1);
+    const float t = add_(add_(t0, t1), add_(u0, u1));
     float o[3];
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
-        float q[4];
-#pragma unroll
-        for (int r = 0; r < 4; r++) q[r] = __shfl_sync(0xffffffffu, t, 4 * c + r);
-        o[c] = add_(add_(q[0], q[2]), add_(q[1], q[3]));
-    }
+    for (int c = 0; c < 3; c++) o[c] = add_(__shfl_sync(0xffffffffu, t, 2 * c), __shfl_sync(0xffffffffu, t, 2 * c + 1));
     return mk3(o[0], o[1], o[2]);
 }
 
 // Attitude rows and body rates for every warp, one vector per lane.
 __device__ __forceinline__ void wide_put_rot(WideSmem& sm, int lane, vec3 r0, vec3 r1, vec3 r2, vec3 w) {
-    if (lane != 0) return;
     sm.rows[0] = make_float4(r0.x, r0.y, r0.z, r1.x);
     sm.rows[1] = make_float4(r1.y, r1.z, r2.x, r2.y);
-    sm.rows[2] = make_float4(r2.z, 0.0f, 0.0f, 0.0f);
-    sm.rate[0] = make_float4(w.x, w.x, w.y, w.y);
-    sm.rate[1] = make_float4(w.z, w.z, -w.x, -w.x);
-    sm.rate[2] = make_float4(-w.y, -w.y, -w.z, -w.z);
+    sm.rows[2] = make_float4(r2.z, w.x, w.y, w.z);
 }
 
 template <bool GRAD>
@@ -183,38 +182,40 @@ __global__ void __launch_bounds__(32 * kWideWarps, 4) k_flight_wide(FlightArgs a
         int to_ck = GRAD ? a.grad_K - step % a.grad_K : 0, ck_i = GRAD ? step / a.grad_K : 0;
         int to_clock = kChunk - step % kChunk;      // steps to the clock's restart
         const int at = (lane & 3) * 8 + (lane >> 2);
-        auto fly = [&](auto two_passes) {
+        auto fly = [&](auto two_passes, auto warp_of) {
             constexpr bool TWO = decltype(two_passes)::value;
+            constexpr int w = decltype(warp_of)::value, w1 = (w + 1) % 3, w2 = (w + 2) % 3;
             constexpr int NP = TWO ? kWidePasses : kWideWarps;
             for (;; step++) {
                 block_sync();
-                const float4 air = sm.air, m0 = sm.rows[0], m1 = sm.rows[1], u0 = sm.rate[0], u1 = sm.rate[1], u2 = sm.rate[2];
-                const float m2 = sm.rows[2].x;
+                const float4 air = sm.air, m0 = sm.rows[0], m1 = sm.rows[1], m2 = sm.rows[2];
                 over = __float_as_int(air.w);
-                const vec3 r0 = mk3(m0.x, m0.y, m0.z), r1 = mk3(m0.w, m1.x, m1.y), r2 = mk3(m1.z, m1.w, m2);
+                const vec3 r0 = mk3(m0.x, m0.y, m0.z), r1 = mk3(m0.w, m1.x, m1.y), r2 = mk3(m1.z, m1.w, m2.x);
                 const vec3 vb = fast_body(r0, r1, r2, mk3(air.x, air.y, air.z));
                 PairConst k;
                 k.vbx = bc(vb.x); k.vby = bc(vb.y); k.vbz = bc(vb.z);
-                k.wbx = pk(u0.x, u0.y); k.wby = pk(u0.z, u0.w); k.wbz = pk(u1.x, u1.y);
-                k.nwbx = pk(u1.z, u1.w); k.nwby = pk(u2.x, u2.y); k.nwbz = pk(u2.z, u2.w);
+                k.wbx = bc(m2.y); k.wby = bc(m2.z); k.wbz = bc(m2.w);
+                k.nwbx = bc(-m2.y); k.nwby = bc(-m2.z); k.nwbz = bc(-m2.w);
                 k.k19 = c_k19; k.cf = bc(fc.skin_cf); k.tiny = c_tiny; k.mone = c_mone;
-                f2 nx, ny, nz;
+                f2 nx, ny, nz, mx, my, mz;
                 pair_force(q0.rbx, q0.rby, q0.rbz, q0.ak, q0.nbx, q0.nby, q0.nbz, k, fc.skin_cf, nx, ny, nz);
-                sm.nf[w][0][lane] = nx; sm.nf[w][1][lane] = ny; sm.nf[w][2][lane] = nz;
+                sm.nf_xy[w][lane] = make_ulonglong2(nx, ny); sm.nf_z[w][lane] = nz;
                 if (TWO) {
-                    pair_force(q1.rbx, q1.rby, q1.rbz, q1.ak, q1.nbx, q1.nby, q1.nbz, k, fc.skin_cf, nx, ny, nz);
-                    sm.nf[w + kWideWarps][0][lane] = nx; sm.nf[w + kWideWarps][1][lane] = ny;
-                    sm.nf[w + kWideWarps][2][lane] = nz;
+                    pair_force(q1.rbx, q1.rby, q1.rbz, q1.ak, q1.nbx, q1.nby, q1.nbz, k, fc.skin_cf, mx, my, mz);
+                    sm.nf_xy[w + kWideWarps][lane] = make_ulonglong2(mx, my); sm.nf_z[w + kWideWarps][lane] = mz;
                 }
                 if (over) break;  // tested here, off the chain: the state is one step too far on
                 block_sync();
-                f2 fn = sm.nf[0][w][lane];
-                f2 tq = mul2(arm2[0], sm.nf[0][w1][lane]), tp = mul2(arm1[0], sm.nf[0][w2][lane]);
+                f2 fn, tq, tp;
 #pragma unroll
-                for (int n = 1; n < NP; n++) {
-                    fn = add2(fn, sm.nf[n][w][lane]);
-                    tq = fma2(arm2[n], sm.nf[n][w1][lane], tq);
-                    tp = fma2(arm1[n], sm.nf[n][w2][lane], tp);
+                for (int n = 0; n < NP; n++) {  // this warp's own passes from its registers
+                    f2 x, y, z;
+                    if (n == w) { x = nx; y = ny; z = nz; }
+                    else if (n == w + kWideWarps) { x = mx; y = my; z = mz; }
+                    else { const ulonglong2 xy = sm.nf_xy[n][lane]; x = xy.x; y = xy.y; z = sm.nf_z[n][lane]; }
+                    fn = n ? add2(fn, axis(x, y, z, w)) : axis(x, y, z, w);
+                    tq = n ? fma2(arm2[n], axis(x, y, z, w1), tq) : mul2(arm2[0], axis(x, y, z, w1));
+                    tp = n ? fma2(arm1[n], axis(x, y, z, w2), tp) : mul2(arm1[0], axis(x, y, z, w2));
                 }
                 float e, o, e2, o2;
                 upk(fn, e, o);
@@ -224,7 +225,7 @@ __global__ void __launch_bounds__(32 * kWideWarps, 4) k_flight_wide(FlightArgs a
                 const bool mark = GRAD && --to_ck == 0;
                 if (mark) { to_ck = a.grad_K; ++ck_i; }
                 FlightState* at_ck = GRAD ? reinterpret_cast<FlightState*>(ck + (size_t)ck_i * 16) : nullptr;
-                if (w == 0) {
+                if constexpr (w == 0) {
                     const vec3 gyro = fast_gyro(fc, st.wb);
                     block_sync();
                     fast_rotate(fc, gyro, wide_fold(sm, 3, lane), st.wb, st.q);
@@ -233,7 +234,7 @@ __global__ void __launch_bounds__(32 * kWideWarps, 4) k_flight_wide(FlightArgs a
                     wide_put_rot(sm, lane, n0, n1, n2, st.wb);
                     // a flight that ends here leaves its checkpoint unread
                     if (mark && lane == 0) { at_ck->q = st.q; at_ck->wb = st.wb; }
-                } else if (w == 1) {
+                } else if constexpr (w == 1) {
                     st.t = add_(st.t, PE_DT);
                     if (--to_clock == 0) {  // as the next step starts: the clock restarts every 600 steps
                         to_clock = kChunk;
@@ -246,9 +247,9 @@ __global__ void __launch_bounds__(32 * kWideWarps, 4) k_flight_wide(FlightArgs a
                     fast_translate(fc, mk3(dot_(r0, Fb), dot_(r1, Fb), dot_(r2, Fb)), st.vel, st.pos);
                     const vec3 wind = wind_lanes(st.pos, tt, wind_of, fc.gust, fc.base_x, fc.base_y);
                     const int now = fast_over(st.pos, st.vel, step, a.max_steps) ? 1 : (step + 1 >= end ? 2 : 0);
+                    sm.air = make_float4(sub_(st.vel.x, wind.x), sub_(st.vel.y, wind.y), sub_(st.vel.z, wind.z),
+                                         __int_as_float(now));
                     if (lane == 0) {
-                        sm.air = make_float4(sub_(st.vel.x, wind.x), sub_(st.vel.y, wind.y), sub_(st.vel.z, wind.z),
-                                             __int_as_float(now));
                         if (mark) {
                             at_ck->pos = st.pos; at_ck->vel = st.vel; at_ck->t = st.t;
                             at_ck->step = 0; at_ck->pad = 0;
@@ -267,7 +268,12 @@ __global__ void __launch_bounds__(32 * kWideWarps, 4) k_flight_wide(FlightArgs a
                 }
             }
         };
-        if (two) fly(std::true_type{}); else fly(std::false_type{});
+        auto as_warp = [&](auto two_passes) {
+            if (w == 0) fly(two_passes, std::integral_constant<int, 0>{});
+            else if (w == 1) fly(two_passes, std::integral_constant<int, 1>{});
+            else fly(two_passes, std::integral_constant<int, 2>{});
+        };
+        if (two) as_warp(std::true_type{}); else as_warp(std::false_type{});
         float fit = 0.0f;
         int kind = 0;
         if (over == 1 && w == 1)

@@ -106,13 +106,13 @@ int flight_fast_blocks_per_sm(const FlightShape& sh);
 cudaError_t launch_flight_fast(const FlightArgs& a, const FlightShape& sh, int grid, cudaStream_t s);
 // Which kernels fly a batch in the default shape (results do not depend on it), by flights per SM.
 // Measured on GB300, milliseconds for pop x 8 with the launch's last 6 flights per SM handed over:
-//   flights per SM            8     14     27     37     54    108    431
-//   a block per flight     0.78   1.24   1.88   2.36   3.41   6.10   23.3
-//   32 lanes, hand-over    0.82   1.02   1.39   1.76   2.32   3.92      -
-//   four per warp, same    0.87   1.21   1.50     -    2.08   3.36   10.8
-// Hand-over at 2, 4, 8 and 12 flights per SM: 2.22, 2.07, 2.06, 2.10 ms at 54; none: 2.74.
-constexpr long long kWideFlights = 6;    // per SM: at most this many take a block each
-constexpr long long kLanesFlights = 32;  // at most this many 32 lanes each, more four per warp
+//   flights per SM            8     10     12     14     21     27     32     37     54    108    431
+//   a block per flight     0.65   0.73   0.94   1.05      -      -      -      -      -      -      -
+//   32 lanes, hand-over    0.72   0.80   0.89   0.94   1.14   1.32   1.56   1.67   2.24   3.85   14.1
+//   four per warp, same       -      -      -   1.02   1.17   1.29   1.44   1.52   1.89   3.14   10.1
+// Hand-over at 4, 6, 8 and 10 flights per SM: 1.89, 1.89, 1.92, 2.06 ms at 54, 0.84, 0.80, 0.80, 1.02 at 10.
+constexpr long long kWideFlights = 10;   // per SM: at most this many take a block each
+constexpr long long kLanesFlights = 24;  // at most this many 32 lanes each, more four per warp
 constexpr int kHandOver = 6;             // the last flights per SM go on with a block each
 constexpr long long kGradLanesFlights = 192;
 

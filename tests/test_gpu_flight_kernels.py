@@ -34,7 +34,8 @@ def _same(torch, pe, G, seeds, **kw):
         assert np.array_equal(a, b), (name, int((a != b).sum()))
 
 
-@pytest.mark.parametrize("per_sm, extra", [(0, 1), (0, 3), (1, 0), (8, -1), (8, 0), (8, 1), (14, 5), (32, 0), (32, 1), (50, 7)])
+@pytest.mark.parametrize("per_sm, extra", [(0, 1), (0, 3), (1, 0), (8, -1), (8, 0), (8, 1), (10, 0), (10, 1), (14, 5),
+                                            (24, 0), (24, 1), (32, 0), (32, 1), (50, 7)])
 def test_default_kernels_at_their_edges(cuda, pe, oracle, per_sm, extra):
     n = per_sm * cuda.cuda.get_device_properties(0).multi_processor_count + extra
     G = oracle.grand(400 + n, n)
