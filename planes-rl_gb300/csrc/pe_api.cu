@@ -636,7 +636,7 @@ int pe_grad(pe_engine* e, const float* d_genomes, int pop, const int* h_seeds, i
     // kAdjBytes, or cannot be had, the serial kernels run, as with PE_GRAD_GROUP = 0 (one flight per
     // block) or 2 (shared blocks).  PE_GRAD_STEPS in the environment lowers kAdjSteps: longer flights
     // take the one-flight kernel (gradients within ~1e-6).  Measured at 256 x 8: 4.03 ms per call with
-    // the serial kernels, 3.32 ms so; at 64 x 8: 2.63 and 1.63 ms.
+    // the serial kernels, 3.25 ms so; at 64 x 8: 2.63 and 1.40 ms.
     const char* steps_env = getenv("PE_GRAD_STEPS");
     const int want_steps = steps_env ? std::max(1, std::min(kAdjSteps, atoi(steps_env))) : kAdjSteps;
     const int rec_steps = (std::min(want_steps, max_steps) + 31) / 32 * 32;

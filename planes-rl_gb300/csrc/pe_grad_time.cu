@@ -11,7 +11,7 @@
 //                   step as a 13 x 10 matrix, column by column through the model's own adjoint functions;
 //   k_adj_chain     a warp per flight, a component per lane: ten shuffles and ten FMAs a step, no barrier;
 //                   leaves the adjoint of every state;
-//   k_adj_panels    block per 512 steps of a flight, a pair or two per lane: the panels' own adjoints and the
+//   k_adj_panels    block per 128 steps of a flight, a pair or two per lane: the panels' own adjoints and the
 //                   mass properties', sums over steps that no longer feed the chain.
 // With v = vb + w x r, B = [I; [r]x] and the panel force f = -(na n + nv v), na and nv functions of v,
 //   d(na)/dv = alpha n + beta v,  d(nv)/dv = gamma v,
@@ -23,8 +23,8 @@
 // Built without fast math, as pe_grad.cu.
 //
 // Measured (GB300, 256 x 8 x 3600 / 64 x 8 x 7200): states 0.05 / 0.04 ms, Jacobians 0.94 / 0.29, chain
-// 0.10 / 0.08 (with the model's adjoint in the chain, eight lanes a flight: 0.74 / 0.66), panels 0.81 /
-// 0.46; the call 4.03 -> 3.32 ms and 2.63 -> 1.63 ms.  The Jacobians and the panels are bound by register
+// 0.10 / 0.08 (with the model's adjoint in the chain, eight lanes a flight: 0.74 / 0.66), panels 0.77 /
+// 0.27 (512 steps a block: 0.81 / 0.46, for want of blocks); the call 4.03 -> 3.25 ms and 2.63 -> 1.40 ms.  The Jacobians and the panels are bound by register
 // reads (a scalar FMA of three registers takes two cycles of the two banks, a packed one three), not by
 // the pipe: 163 instructions per panel and 32 steps take 224 cycles.
 #include <cuda_runtime.h>

@@ -163,7 +163,7 @@ constexpr int kGradCounters = 9;
 // matrices per 32 of them, for flights of at most kAdjSteps steps, and adds the plane's adjoints in parts
 // of kAdjPart steps; it is taken where the records fit kAdjBytes.
 constexpr int kAdjEnt = 24, kAdjChunk = 4292;
-constexpr int kAdjSteps = 3072, kAdjPart = 512;
+constexpr int kAdjSteps = 3072, kAdjPart = 128;  // 512 / 256 / 128 / 64: 1.62, 1.45, 1.40, 1.41 ms at 64 x 8, 3.32, 3.31, 3.25, 3.26 at 256 x 8
 constexpr size_t kAdjBytes = 8ull << 30;
 
 struct GradArgs {
