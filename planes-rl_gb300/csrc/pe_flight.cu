@@ -88,7 +88,7 @@ struct RefBlock {
 };
 
 // What the integrator needs of FlightConst, next to the panels'.
-struct RefConst {
+struct alignas(16) RefConst {
     float I[6], invI[9], pad0;                                      // the rotation's: four float4
     float mass, invmass, phase, gust, base_x, base_y, pad1, pad2;   // the translation's: two
 };
