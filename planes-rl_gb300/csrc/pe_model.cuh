@@ -305,17 +305,15 @@ struct MassProps {
     float invI[9];
 };
 
-// src/common.h:311-365 by one warp.  The lanes compute every triangle's terms in parallel into
-// shared memory (T: kMpTerms x kNtMax floats, term k of triangle i at T[k * kNtMax + i]); then each
-// sum is one lane's, added in emission order with the multiply-adds of a one-thread loop, so the sums
-// round exactly as the reference's serial loop does.  (All on lane 0, the chains shared its issue
-// slots: 17.1 us a plane alone and 207 us for 8,192, now 14.2 and 174.)  Two passes, as
-// in the reference: the centre of mass first, then the inertia about it.  The 3x3 inverse that the flight never reads (the
-// print-varied inverse replaces it) is taken in FP64.  Called by all 32 lanes; *mp on lane 0.
+// src/common.h:311-365 by a block of threads 0 .. threads - 1.  They compute every triangle's terms in
+// parallel into shared memory (T: kMpTerms x kNtMax floats, term k of triangle i at T[k * kNtMax + i]); then
+// each sum is one lane's of warp 0, added in emission order with the multiply-adds of a one-thread loop, so
+// the sums round exactly as the reference's serial loop does.  Two passes, as in the reference: the centre of
+// mass first (mass_first: terms, mass_com: sums), then the inertia about it (mass_second, mass_inertia).
+// The 3x3 inverse that the flight never reads (the print-varied inverse replaces it) is taken in FP64.
 constexpr int kMpTerms = 15;
-static __device__ __noinline__ void mass_props(GenomeRef g, const vec3* V, const Topo& tp, int lane, float* T,
-                                               float* s_c, MassProps* mp) {
-    for (int i = lane; i < tp.nt; i += 32) {
+__device__ __forceinline__ void mass_first(const vec3* V, const Topo& tp, int tid, int threads, float* T) {
+    for (int i = tid; i < tp.nt; i += threads) {
         int ia, ib, ic; mesh_tri(tp, i, &ia, &ib, &ic);
         vec3 a = V[ia], b = V[ib], d = V[ic];
         float A = 0.5f * vlen(vcross(vsub(b, a), vsub(d, a)));
@@ -323,7 +321,9 @@ static __device__ __noinline__ void mass_props(GenomeRef g, const vec3* V, const
         vec3 ct = vscl(vadd(vadd(a, b), d), 1.0f / 3);
         T[i] = mi; T[kNtMax + i] = ct.x; T[2 * kNtMax + i] = ct.y; T[3 * kNtMax + i] = ct.z;
     }
-    __syncwarp();
+}
+// By warp 0: mass with the nose ballast to s_c[3], centre of mass to s_c[0..2], the ballast's mass to s_c[4].
+__device__ __forceinline__ void mass_com(GenomeRef g, const Topo& tp, int lane, const float* T, float* s_c) {
     // lane 0 the mass, lanes 1..3 the mass moments: a chain of one multiply-add per triangle each
     const float* tc = T + min(lane, 3) * kNtMax;
     float sum = 0;
@@ -336,18 +336,17 @@ static __device__ __noinline__ void mass_props(GenomeRef g, const vec3* V, const
     }
     float m = __shfl_sync(0xffffffffu, sum, 0), mn = 0;
     vec3 c = mk3(__shfl_sync(0xffffffffu, sum, 1), __shfl_sync(0xffffffffu, sum, 2), __shfl_sync(0xffffffffu, sum, 3));
-    vec3 np = mk3(0, 0, 0);
     if (lane == 0) {
         float shell_m = m;
-        np = mk3(0.5f * g[G_CHORD], 0, 0);
+        vec3 np = mk3(0.5f * g[G_CHORD], 0, 0);
         mn = g[G_NOSE] * shell_m;
         m += mn; c = vadd(c, vscl(np, mn));
         c = vscl(c, 1.0f / m);
-        s_c[0] = c.x; s_c[1] = c.y; s_c[2] = c.z;
+        s_c[0] = c.x; s_c[1] = c.y; s_c[2] = c.z; s_c[3] = m; s_c[4] = mn;
     }
-    __syncwarp();
-    c = mk3(s_c[0], s_c[1], s_c[2]);
-    for (int i = lane; i < tp.nt; i += 32) {
+}
+__device__ __forceinline__ void mass_second(const vec3* V, const Topo& tp, int tid, int threads, vec3 c, float* T) {
+    for (int i = tid; i < tp.nt; i += threads) {
         int ia, ib, ic; mesh_tri(tp, i, &ia, &ib, &ic);
         vec3 a = V[ia], b = V[ib], d = V[ic];
         float A = 0.5f * vlen(vcross(vsub(b, a), vsub(d, a)));
@@ -371,7 +370,10 @@ static __device__ __noinline__ void mass_props(GenomeRef g, const vec3* V, const
         t[10 * kNtMax] = 1.0f - nn.z * nn.z; t[11 * kNtMax] = th * nn.x; t[12 * kNtMax] = th * nn.y;
         t[13 * kNtMax] = nn.y; t[14 * kNtMax] = nn.z;
     }
-    __syncwarp();
+}
+// By warp 0; *mp on lane 0.
+static __device__ __noinline__ void mass_inertia(GenomeRef g, const Topo& tp, int lane, const float* T, const float* s_c,
+                                                 MassProps* mp) {
     // lane k the component I[k]: two multiply-adds per triangle, xx yy zz adding and xy xz yz subtracting
     const int k = min(lane, 5);
     const float* t1 = T + (1 + k) * kNtMax;                      // mi *
@@ -388,10 +390,13 @@ static __device__ __noinline__ void mass_props(GenomeRef g, const vec3* V, const
 #pragma unroll
     for (int q = 0; q < 6; q++) I[q] = __shfl_sync(0xffffffffu, part, q);
     if (lane != 0) return;
+    const float m = s_c[3], mn = s_c[4];
+    const vec3 c = mk3(s_c[0], s_c[1], s_c[2]);
     {
-        vec3 r = vsub(np, c);
-        I[0] += mn * (r.y * r.y + r.z * r.z); I[1] += mn * (r.x * r.x + r.z * r.z);
-        I[2] += mn * (r.x * r.x + r.y * r.y); I[3] -= mn * r.x * r.y;
+        vec3 r = vsub(mk3(0.5f * g[G_CHORD], 0, 0), c);
+        const float yy = __fmul_rn(r.y, r.y), zz = __fmul_rn(r.z, r.z);  // fused as in a one-thread loop
+        I[0] += mn * __fadd_rn(yy, zz); I[1] += mn * __fmaf_rn(r.x, r.x, zz);
+        I[2] += mn * __fmaf_rn(r.x, r.x, yy); I[3] -= mn * r.x * r.y;
         I[4] -= mn * r.x * r.z; I[5] -= mn * r.y * r.z;
     }
     float reg = 1e-9f;

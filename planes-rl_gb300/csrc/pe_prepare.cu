@@ -5,10 +5,10 @@
 //                 exclusive scan, block totals out.
 //   k_scan_tot    exclusive scan of the block totals (one block, 1024 at a time); also the
 //                 grand total.
-//   k_mesh        one warp per plane: lanes evaluate the mesh vertices in parallel into shared
+//   k_mesh        a block per plane: threads evaluate the mesh vertices in parallel into shared
 //                 memory and every triangle's mass-property terms likewise; then each sum is one
 //                 lane's, in emission order (the reference's order, so the sums round identically);
-//                 lanes write the COM-relative panel SoA into the plane's exact prefix range.
+//                 the COM-relative panel SoA goes into the plane's exact prefix range.
 // HBM traffic is small (140 B genome in, 32 B per panel out); the cost is the ordered sums.
 #include "pe_internal.cuh"
 
@@ -86,63 +86,78 @@ __global__ void __launch_bounds__(1024) k_scan_tot(int* block_sum, int nblocks, 
     if (threadIdx.x == 0) *total = carry;
 }
 
-constexpr int kMeshWarps = 2;  // shared memory: 2 x (15 x 344 mass-property terms + 241 vertices)
+// A block per plane: all threads take the vertices and the sums' terms; then warp 0 adds in order while
+// warp 1 finds the extent, and once more while the others write the panels.  Bound by the two chains of
+// ordered sums and what leads up to them.  The preparation's launches together, with a warp per plane (two
+// per block of 46 KB, eight per SM) and so: 21.5 -> 17.5 us for one plane, 31 -> 23 for 8 to 128, 88 -> 69 for
+// 3,001, 184 -> 141 for 8,192, 1,920 -> 1,430 for 100,000.
+constexpr int kMeshThreads = 128;
 
-__global__ void __launch_bounds__(kMeshWarps * 32) k_mesh(PrepArgs a) {
-    __shared__ float s_g[kMeshWarps][kGenomeN + 1];
-    __shared__ vec3 s_v[kMeshWarps][kNvMax];
-    __shared__ float s_com[kMeshWarps][4];
-    __shared__ float s_terms[kMeshWarps][kMpTerms * kNtMax];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int p = blockIdx.x * kMeshWarps + w;
-    if (p >= a.pop) return;  // warp-uniform; no block barrier follows
-    const float* src = a.genomes + (size_t)p * kGenomeN;
-    for (int i = lane; i < kGenomeN; i += 32) s_g[w][i] = src[i];
-    __syncwarp();
-    GenomeRef g{s_g[w]};
+__global__ void __launch_bounds__(kMeshThreads, 8) k_mesh(PrepArgs a) {
+    __shared__ float s_g[kGenomeN + 1];
+    __shared__ vec3 s_v[kNvMax];
+    __shared__ float s_com[5];
+    __shared__ float s_terms[kMpTerms * kNtMax];
+    __shared__ int s_nt;
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+    const int p = blockIdx.x;
+    if (tid < kGenomeN) s_g[tid] = a.genomes[(size_t)p * kGenomeN + tid];
+    __syncthreads();
+    GenomeRef g{s_g};
     const Topo tp = topology(g);
-    for (int i = lane; i < tp.nv; i += 32) s_v[w][i] = mesh_vertex(g, tp, i);
-    __syncwarp();
-
-    // mesh extent (min/max are exact in any order), src/common.h:294-307
-    vec3 lo = s_v[w][0], hi = lo;
-    for (int i = lane; i < tp.nv; i += 32) {
-        vec3 v = s_v[w][i];
-        lo.x = fminf(lo.x, v.x); lo.y = fminf(lo.y, v.y); lo.z = fminf(lo.z, v.z);
-        hi.x = fmaxf(hi.x, v.x); hi.y = fmaxf(hi.y, v.y); hi.z = fmaxf(hi.z, v.z);
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        lo.x = fminf(lo.x, __shfl_xor_sync(0xffffffffu, lo.x, o));
-        lo.y = fminf(lo.y, __shfl_xor_sync(0xffffffffu, lo.y, o));
-        lo.z = fminf(lo.z, __shfl_xor_sync(0xffffffffu, lo.z, o));
-        hi.x = fmaxf(hi.x, __shfl_xor_sync(0xffffffffu, hi.x, o));
-        hi.y = fmaxf(hi.y, __shfl_xor_sync(0xffffffffu, hi.y, o));
-        hi.z = fmaxf(hi.z, __shfl_xor_sync(0xffffffffu, hi.z, o));
-    }
-    vec3 ext = vsub(hi, lo);
-    const float lim = PE_PRINT_LIMIT;
-    const int printable = ext.x <= lim && ext.y <= lim && ext.z <= lim;
-    const int nt = printable ? tp.nt : 0;
+    for (int i = tid; i < tp.nv; i += kMeshThreads) s_v[i] = mesh_vertex(g, tp, i);
     const int off = a.pt.off[p] + a.block_sum[p / kScanBlock];
-
-    MassProps mp;
-    mass_props(g, s_v[w], tp, lane, s_terms[w], s_com[w], &mp);
-    if (lane == 0) {
-        float* o = a.pt.mp + (size_t)p * kMpN;
-        o[0] = mp.mass; o[1] = mp.invmass; o[2] = mp.com.x; o[3] = mp.com.y; o[4] = mp.com.z;
-        for (int k = 0; k < 6; k++) o[5 + k] = mp.I[k];
-        for (int k = 0; k < 9; k++) o[11 + k] = mp.invI[k];
-        s_com[w][0] = mp.com.x; s_com[w][1] = mp.com.y; s_com[w][2] = mp.com.z;
-        a.pt.nt[p] = nt;
-        a.pt.ext[p] = make_float4(ext.x, ext.y, ext.z, (float)tp.nt);
+    __syncthreads();
+    mass_first(s_v, tp, tid, kMeshThreads, s_terms);
+    __syncthreads();
+    if (w == 0) {
+        mass_com(g, tp, lane, s_terms, s_com);
+    } else if (w == 1) {
+        // mesh extent (min/max are exact in any order), src/common.h:294-307
+        vec3 lo = s_v[0], hi = lo;
+        for (int i = lane; i < tp.nv; i += 32) {
+            vec3 v = s_v[i];
+            lo.x = fminf(lo.x, v.x); lo.y = fminf(lo.y, v.y); lo.z = fminf(lo.z, v.z);
+            hi.x = fmaxf(hi.x, v.x); hi.y = fmaxf(hi.y, v.y); hi.z = fmaxf(hi.z, v.z);
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            lo.x = fminf(lo.x, __shfl_xor_sync(0xffffffffu, lo.x, o));
+            lo.y = fminf(lo.y, __shfl_xor_sync(0xffffffffu, lo.y, o));
+            lo.z = fminf(lo.z, __shfl_xor_sync(0xffffffffu, lo.z, o));
+            hi.x = fmaxf(hi.x, __shfl_xor_sync(0xffffffffu, hi.x, o));
+            hi.y = fmaxf(hi.y, __shfl_xor_sync(0xffffffffu, hi.y, o));
+            hi.z = fmaxf(hi.z, __shfl_xor_sync(0xffffffffu, hi.z, o));
+        }
+        vec3 ext = vsub(hi, lo);
+        const float lim = PE_PRINT_LIMIT;
+        const int printable = ext.x <= lim && ext.y <= lim && ext.z <= lim;
+        if (lane == 0) {
+            s_nt = printable ? tp.nt : 0;
+            a.pt.nt[p] = s_nt;
+            a.pt.off[p] = off;
+            a.pt.ext[p] = make_float4(ext.x, ext.y, ext.z, (float)tp.nt);
+        }
     }
-    __syncwarp();
-    if (lane == 0) a.pt.off[p] = off;
-    const vec3 com = mk3(s_com[w][0], s_com[w][1], s_com[w][2]);
+    __syncthreads();
+    const vec3 com = mk3(s_com[0], s_com[1], s_com[2]);
+    mass_second(s_v, tp, tid, kMeshThreads, com, s_terms);
+    __syncthreads();
+    if (w == 0) {
+        MassProps mp;
+        mass_inertia(g, tp, lane, s_terms, s_com, &mp);
+        if (lane == 0) {
+            float* o = a.pt.mp + (size_t)p * kMpN;
+            o[0] = mp.mass; o[1] = mp.invmass; o[2] = mp.com.x; o[3] = mp.com.y; o[4] = mp.com.z;
+            for (int k = 0; k < 6; k++) o[5 + k] = mp.I[k];
+            for (int k = 0; k < 9; k++) o[11 + k] = mp.invI[k];
+        }
+        return;
+    }
     // COM-relative panels, src/sim.cu:40-48
-    for (int t = lane; t < nt; t += 32) {
+    const int nt = s_nt;
+    for (int t = tid - 32; t < nt; t += kMeshThreads - 32) {
         int ia, ib, ic; mesh_tri(tp, t, &ia, &ib, &ic);
-        vec3 pa = vsub(s_v[w][ia], com), pb = vsub(s_v[w][ib], com), pcv = vsub(s_v[w][ic], com);
+        vec3 pa = vsub(s_v[ia], com), pb = vsub(s_v[ib], com), pcv = vsub(s_v[ic], com);
         vec3 nrm = vcross(vsub(pb, pa), vsub(pcv, pa));
         float A = 0.5f * vlen(nrm);
         vec3 ct = vscl(vadd(vadd(pa, pb), pcv), 1.0f / 3);
@@ -157,7 +172,7 @@ cudaError_t set_station_mode(int ieee) {
     return cudaMemcpyToSymbol(c_station_ieee, &v, sizeof(int));
 }
 
-// A small batch's preparation is its launches: without the scan's, 2 of 17 us at one genome; from some
+// A small batch's preparation is its launches: without the scan's, 2 of 19 us at one genome; from some
 // hundreds on k_mesh and the flights hide it.
 constexpr int kScanAlone = 128;
 static_assert(kScanAlone <= kScanBlock, "one block counts them");
@@ -167,7 +182,7 @@ int launch_prepare(const PrepArgs& a, int* d_total, cudaStream_t s) {
     const bool alone = a.pop <= kScanAlone;
     k_topo_scan<<<nb, kScanBlock, 0, s>>>(a, alone ? d_total : nullptr);
     if (!alone) k_scan_tot<<<1, 1024, 0, s>>>(a.block_sum, nb, d_total);
-    k_mesh<<<(a.pop + kMeshWarps - 1) / kMeshWarps, kMeshWarps * 32, 0, s>>>(a);
+    k_mesh<<<a.pop, kMeshThreads, 0, s>>>(a);
     return alone ? 2 : 3;
 }
 
