@@ -120,6 +120,8 @@ struct pe_engine {
     // host-buffer path
     DevBuf<float> g_dev, dist_dev, scores_dev;
     DevBuf<int> steps_dev;
+    DevBuf<float> stage_dev;   // a small call's distances, steps and scores, one after the other
+    std::vector<float> stage;  // where they come back in one copy
     DevBuf<float> audit_stats;  // pe_audit's 13 statistics
     // timing
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -347,6 +349,8 @@ int enqueue_eval(pe_engine* e, const float* d_genomes, int pop, int nseeds, int 
     return PE_OK;
 }
 
+constexpr size_t kStageWords = 32 << 10;  // results that pe_evaluate_population brings back in one copy
+
 int check_seeds(const int* h_seeds, int nseeds) {
     if (!h_seeds || nseeds <= 0) return fail(PE_EINVAL, "seeds must be a non-empty host array");
     return PE_OK;
@@ -499,19 +503,44 @@ int pe_evaluate_population(pe_engine* e, const float* h_genomes, int pop, const 
         if (g_eval_budget.compare_exchange_weak(b, b - 1)) break;
     }
     if (int rc = ensure_device(e)) return rc;
-    const size_t nf = (size_t)pop * nseeds;
+    const size_t nf = (size_t)pop * nseeds, words = 2 * nf + pop;
     PE_CUDA(e->g_dev.ensure((size_t)pop * kGenomeN));
-    PE_CUDA(e->dist_dev.ensure(nf));
-    PE_CUDA(e->steps_dev.ensure(nf));
-    PE_CUDA(e->scores_dev.ensure((size_t)pop));
+    // A copy to pageable memory waits for the stream and is staged by the driver: the results of a small call
+    // come back in one instead of three (one plane x 8: 287 -> 269 us a call; pinned
+    // memory 266, and 100 us on an engine's first call).  Results beyond kStageWords hide the copies.
+    const bool staged = words <= kStageWords;
+    float *dist = nullptr, *scores = nullptr;
+    int* steps = nullptr;
+    if (staged) {
+        PE_CUDA(e->stage_dev.ensure(kStageWords));
+        e->stage.resize(kStageWords);
+        dist = e->stage_dev.p;
+        steps = reinterpret_cast<int*>(dist + nf);
+        scores = dist + 2 * nf;
+    } else {
+        PE_CUDA(e->dist_dev.ensure(nf));
+        PE_CUDA(e->steps_dev.ensure(nf));
+        PE_CUDA(e->scores_dev.ensure((size_t)pop));
+        dist = e->dist_dev.p;
+        steps = e->steps_dev.p;
+        scores = e->scores_dev.p;
+    }
     cudaStream_t s = nullptr;
     PE_CUDA(cudaMemcpyAsync(e->g_dev.p, h_genomes, sizeof(float) * kGenomeN * pop, cudaMemcpyHostToDevice, s));
-    int rc = pe_eval_batch(e, e->g_dev.p, pop, h_seeds, nseeds, vary, max_steps, e->dist_dev.p, e->steps_dev.p,
-                           h_scores ? e->scores_dev.p : nullptr, s);
+    int rc = pe_eval_batch(e, e->g_dev.p, pop, h_seeds, nseeds, vary, max_steps, dist, steps, h_scores ? scores : nullptr, s);
     if (rc != PE_OK) return rc;
-    if (h_dist) PE_CUDA(cudaMemcpyAsync(h_dist, e->dist_dev.p, sizeof(float) * nf, cudaMemcpyDeviceToHost, s));
-    if (h_steps) PE_CUDA(cudaMemcpyAsync(h_steps, e->steps_dev.p, sizeof(int) * nf, cudaMemcpyDeviceToHost, s));
-    if (h_scores) PE_CUDA(cudaMemcpyAsync(h_scores, e->scores_dev.p, sizeof(float) * pop, cudaMemcpyDeviceToHost, s));
+    if (staged) {
+        const float* got = e->stage.data();
+        PE_CUDA(cudaMemcpyAsync(e->stage.data(), dist, sizeof(float) * words, cudaMemcpyDeviceToHost, s));
+        PE_CUDA(cudaStreamSynchronize(s));
+        if (h_dist) memcpy(h_dist, got, sizeof(float) * nf);
+        if (h_steps) memcpy(h_steps, got + nf, sizeof(int) * nf);
+        if (h_scores) memcpy(h_scores, got + 2 * nf, sizeof(float) * pop);
+        return PE_OK;
+    }
+    if (h_dist) PE_CUDA(cudaMemcpyAsync(h_dist, dist, sizeof(float) * nf, cudaMemcpyDeviceToHost, s));
+    if (h_steps) PE_CUDA(cudaMemcpyAsync(h_steps, steps, sizeof(int) * nf, cudaMemcpyDeviceToHost, s));
+    if (h_scores) PE_CUDA(cudaMemcpyAsync(h_scores, scores, sizeof(float) * pop, cudaMemcpyDeviceToHost, s));
     PE_CUDA(cudaStreamSynchronize(s));
     return PE_OK;
 }

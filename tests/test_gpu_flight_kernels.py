@@ -162,3 +162,21 @@ def test_reference_order_blocks(cuda, pe, oracle, pop, S, max_steps, chunk):
     for p in range(min(pop, 5)):
         a = fly(G[p:p + 1], 7200)
         assert np.array_equal(a[0], d[p * S:(p + 1) * S]) and np.array_equal(a[1], st[p * S:(p + 1) * S])
+
+
+@pytest.mark.parametrize("pop,S", [(1, 1), (3, 5), (32, 511), (32, 512)])  # results in one copy, and just beyond
+@pytest.mark.parametrize("want", ["dist", "steps", "scores", "all"])
+def test_host_results(cuda, pe, oracle, pop, S, want):
+    torch = cuda
+    G, seeds = oracle.grand(23, pop), list(range(5, 5 + S))
+    e = pe.Engine(0)
+    d, st, sc = torch.empty(pop * S, device="cuda"), torch.empty(pop * S, dtype=torch.int32, device="cuda"), torch.empty(pop, device="cuda")
+    e.eval_batch(torch.from_numpy(G).cuda(), pop, seeds, 0, 40, d, st, sc)
+    torch.cuda.synchronize()
+    ref = {"dist": d, "steps": st, "scores": sc}
+    for _ in range(2):
+        out = e.evaluate_population(G, seeds, max_steps=40, **{"want_" + k: want in (k, "all") for k in ref})
+        assert set(out) == {k for k in ref if want in (k, "all")}
+        for k, v in out.items():
+            assert np.array_equal(v, ref[k].cpu().numpy())
+    e.close()
