@@ -9,10 +9,9 @@
 //
 //   k_obj_prepare   one block per plane: mesh, printability, mass properties (two passes over
 //                   the triangles with block reductions) and panels, in T.
-//   k_obj_forward   one block of kObjW warps per flight, persistent over a work queue: print
+//   k_obj_forward   few flights in FP32: one block of kObjW warps per flight, persistent over a work queue: print
 //                   variation, staging, release and the flight; writes the smoothed distance.
-//   k_obj_forward4  the same with four flights per block, for FP64.
-//   k_obj_flights   four flights per block with their integrators in one warp, for many flights in FP32.
+//   k_obj_flights   four flights per block with their integrators in one warp, for many flights and FP64.
 //   k_obj_weights   one block per plane: the tail-aware objective of its distances.
 #include <cuda_runtime.h>
 
@@ -121,9 +120,9 @@ __global__ void __launch_bounds__(kObjThreads) k_obj_prepare(ObjArgs a) {
     }
 }
 
-// ------------------------------------------------------------------ flights in T
-template <class T>
+// ------------------------------------------------------------------ few flights in FP32
 __global__ void __launch_bounds__(32 * kObjW) k_obj_forward(ObjArgs a) {
+    using T = float;
     using V3T = pg::V3<T>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* part = reinterpret_cast<T*>(smem_raw);        // [2][kObjW][8]
@@ -214,14 +213,6 @@ __global__ void __launch_bounds__(32 * kObjW) k_obj_forward(ObjArgs a) {
     }
 }
 
-// One of a block's four flights, and the warp's of the same number.
-template <class T>
-struct ObjSlot {
-    T part[kObjW][8];  // each warp's sums of the step's force and torque
-    T pre[8];          // vb xyz, w xyz, skin friction
-    T sp[7 * kNtMax];  // staged panels (SoA)
-};
-
 // The sums over a warp of 24 values per lane (six of each of four flights), transposed: a level halves
 // the values a lane carries, 24 shuffles instead of 120, and each sum follows the xor tree that a
 // butterfly over all lanes would.  Lane 8 m + 4 h + q (q < 3) returns component 3 h + q of flight m.
@@ -245,220 +236,114 @@ __device__ __forceinline__ T warp_sum24(T (&v)[24], int lane) {
     return v[0];
 }
 
-// Four flights per block: all warps take the panels of every flight, each warp its own flight's integrator
-// and gusts, so that a flight-step is a third of the warp instructions.  Two barriers per step and a longer
-// chain, which FP64's panels outweigh at any number of flights.
-template <class T>
-__global__ void __launch_bounds__(32 * kObjW, 1) k_obj_forward4(ObjArgs a) {
-    using V3T = pg::V3<T>;
-    constexpr int nthr = 32 * kObjW;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    ObjSlot<T>* slot = reinterpret_cast<ObjSlot<T>*>(smem_raw);
-    __shared__ int s_nt[kObjW];  // panels of each slot's flight (0: none)
-    static_assert(kObjW == 4, "warp_sum24 takes four flights");
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int n_flights = a.pop * a.nseeds;
-    ObjSlot<T>& mine = slot[warp];
-    int f = 0, j = 0, to_chunk = 0;
-    bool live = false;
-    pg::FlightP<T> P;
-    pg::St<T> s;
-    pg::Pre<T> pr{};
-    auto publish = [&]() {
-        if (lane == 0) {
-            mine.pre[0] = pr.vb.x; mine.pre[1] = pr.vb.y; mine.pre[2] = pr.vb.z;
-            mine.pre[3] = pr.w.x; mine.pre[4] = pr.w.y; mine.pre[5] = pr.w.z;
-        }
-    };
-    auto next_flight = [&]() {
-        for (;;) {
-            if (lane == 0) f = atomicAdd(a.work, 1);
-            f = __shfl_sync(0xffffffffu, f, 0);
-            live = f < n_flights;
-            if (!live) {
-                if (lane == 0) s_nt[warp] = 0;
-                return;
-            }
-            const int p = f / a.nseeds, si = f - p * a.nseeds;
-            const T* pl = reinterpret_cast<const T*>(a.plane) + (size_t)p * kObjPlaneStride;
-            const int nt = (int)pl[7];
-            if (nt <= 0) {  // does not fit the print volume
-                if (lane == 0) a.dist[f] = -100.0;
-                continue;
-            }
-            const int seed = a.seeds[si] + (a.vary ? p * 7919 : 0);
-            Scenario S;
-            scenario_desc(seed, &S);
-            T sc[kScenN];
-#pragma unroll
-            for (int k = 0; k < kScenN; k++) sc[k] = (T)S.v[k];
-            V3T cg;
-            T sigma, beta[6], I[6];
-#pragma unroll
-            for (int q = 0; q < 6; q++) I[q] = pl[1 + q];
-            pg::printed(sc, pl[0], I, P, &cg, &sigma, beta);
-            P.phase = (T)seed_phase(seed);
-            const T* pc = pl + 8;
-            T* sp = mine.sp;
-            for (int i = lane; i < nt; i += 32) {
-                V3T rb, nb;
-                T ak;
-                pg::stage(pg::v3(pc[i], pc[kNtMax + i], pc[2 * kNtMax + i]), pc[3 * kNtMax + i],
-                          pg::v3(pc[4 * kNtMax + i], pc[5 * kNtMax + i], pc[6 * kNtMax + i]), cg, sc[pg::SC_RHO],
-                          sc[pg::SC_WP], sc[pg::SC_WR], &rb, &nb, &ak);
-                sp[i] = rb.x; sp[kNtMax + i] = rb.y; sp[2 * kNtMax + i] = rb.z;
-                sp[3 * kNtMax + i] = nb.x; sp[4 * kNtMax + i] = nb.y; sp[5 * kNtMax + i] = nb.z;
-                sp[6 * kNtMax + i] = ak;
-            }
-            s = pg::release(sc, P, cg, (V3T*)nullptr, (V3T*)nullptr);
-            pg::step_pre(P, s, pr);
-            publish();
-            if (lane == 0) {
-                mine.pre[6] = P.cf;
-                s_nt[warp] = nt;
-            }
-            j = 0;
-            to_chunk = kChunk;
-            return;
-        }
-    };
-    next_flight();
-    for (;;) {
-        __syncthreads();
-        if (!(s_nt[0] | s_nt[1] | s_nt[2] | s_nt[3])) break;
-        T v[24];
-#pragma unroll
-        for (int m = 0; m < kObjW; m++) {
-            T acc[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
-            const T* pre = slot[m].pre;
-            pg::Pre<T> q;
-            q.vb = pg::v3(pre[0], pre[1], pre[2]);
-            q.w = pg::v3(pre[3], pre[4], pre[5]);
-            const int nt = s_nt[m];
-            const T* sp = slot[m].sp;
-            const T cf = pre[6];
-            for (int i = tid; i < nt; i += nthr) {
-                V3T fo, tq;
-                pg::panel_fwd(q, pg::v3(sp[i], sp[kNtMax + i], sp[2 * kNtMax + i]),
-                              pg::v3(sp[3 * kNtMax + i], sp[4 * kNtMax + i], sp[5 * kNtMax + i]), sp[6 * kNtMax + i],
-                              cf, &fo, &tq);
-                acc[0] += fo.x; acc[1] += fo.y; acc[2] += fo.z;
-                acc[3] += tq.x; acc[4] += tq.y; acc[5] += tq.z;
-            }
-#pragma unroll
-            for (int k = 0; k < 6; k++) v[6 * m + k] = acc[k];
-        }
-        const T total = warp_sum24(v, lane);
-        if ((lane & 3) != 3) slot[lane >> 3].part[warp][3 * ((lane >> 2) & 1) + (lane & 3)] = total;
-        __syncthreads();
-        if (!live) continue;
-        T w[6];
-#pragma unroll
-        for (int k = 0; k < 6; k++) {
-            T t = mine.part[0][k];
-#pragma unroll
-            for (int q = 1; q < kObjW; q++) t += mine.part[q][k];
-            w[k] = t;
-        }
-        const pg::St<T> nx = pg::step_post(P, s, pr, pg::v3(w[0], w[1], w[2]), pg::v3(w[3], w[4], w[5]));
-        T d = T(0);
-        int kind = 0;
-        if (pg::terminate(s, nx, j, a.max_steps, &d, &kind)) {
-            if (lane == 0) a.dist[f] = (double)d;
-            next_flight();
-        } else {
-            s = nx;
-            if (--to_chunk == 0) { s.t = T((double)(j + 1)) * T(pg::kDt); to_chunk = kChunk; }  // src/sim.cu:113
-            j++;
-            pg::step_pre(P, s, pr);
-            publish();
-        }
-    }
-}
-
-// ------------------------------------------------------------------ many flights in FP32
-// Four flights per block as in k_obj_forward4, and one warp turns all four while another moves them and
-// takes their gusts (eight lanes a flight), other warps each step; state and constants stay in shared memory,
-// which leaves 90 registers and five blocks per SM instead of four of 108.  Warp (k + flight) % 4 takes the
-// panels i % 128 / 32 == k of a flight, so a short last round falls on another warp for each of the four.
-// Bound by issue slots.  512 x 8: 2.52 -> 2.24 ms, 1500 x 8: 5.78 -> 4.83 (k_obj_forward4, then this); a
-// lone flight's step takes a fifth longer than with a block of its own.
+// ------------------------------------------------------------------ four flights per block
+// All warps take the panels of every flight; then one warp turns all four flights and another moves them and
+// takes their gusts (eight lanes a flight), other warps each step.  State and constants stay in shared memory,
+// which leaves 90 registers and five blocks per SM in FP32.  Warp (k + flight) % 4 takes the panels
+// i % 128 / 32 == k of a flight, so a short last round falls on another warp for each of the four.  Bound by
+// issue slots (FP32) and the FP64 pipe.  With each warp running its own flight's integrator: FP32 512 x 8
+// 2.52 ms, 1500 x 8 5.78, FP64 512 x 8 86; so 2.24, 4.83 and 72.  A lone FP32 flight's step takes a fifth
+// longer than with a block of its own.
 constexpr int kObjPad = (kNtMax + 31) / 32 * 32;  // staged panels, filled up with empty ones
 
+template <class T>
+struct alignas(16) Vec4 { T x, y, z, w; };
+template <class T>
+struct alignas(2 * sizeof(T)) Vec2 { T x, y; };
+
+template <class T>
 struct ObjBlock {
-    float4 pos_t[kObjW], vel[kObjW], q[kObjW], w[kObjW];
-    float4 cst[6][kObjW];          // ObjConst
-    float4 rows[2][kObjW][3];      // attitude of this step and the next: rows, skin friction in the last place
-    float4 va[kObjW];              // air velocity
-    float4 part[kObjW][2 * kObjW + 1];
+    using V4 = Vec4<T>;
+    V4 pos_t[kObjW], vel[kObjW], q[kObjW], w[kObjW];
+    V4 cst[6][kObjW];          // ObjConst
+    V4 rows[2][kObjW][3];      // attitude of this step and the next: rows, skin friction in the last place
+    V4 va[kObjW];              // air velocity
+    V4 part[kObjW][2 * kObjW + 1];
     int nt[kObjW], flight[kObjW], step[kObjW];
-    float4 rb[kObjW][kObjPad];     // centroid, half the density times the area
-    float2 nxy[kObjW][kObjPad];    // normal
-    float nz[kObjW][kObjPad];
+    V4 rb[kObjW][kObjPad];     // centroid, half the density times the area
+    Vec2<T> nxy[kObjW][kObjPad];    // normal
+    T nz[kObjW][kObjPad];
 };
+template <class T>
 struct alignas(16) ObjConst {
-    float I[6], invI[9], cf;
-    float mass, invmass, gust, phase, base_x, base_y, pad0, pad1;
+    T I[6], invI[9], cf;
+    T mass, invmass, gust, phase, base_x, base_y, pad0, pad1;
 };
-static_assert(sizeof(ObjConst) == 6 * sizeof(float4), "ObjConst is six float4");
+static_assert(sizeof(ObjConst<float>) == 6 * sizeof(Vec4<float>), "ObjConst is six Vec4");
 
 // Sums of products with their fused operations spelled out, so that results do not hang on how the compiler
 // pairs them: a b + c d (+ e f).
-__device__ __forceinline__ float sum2(float a, float b, float c, float d) { return __fmaf_rn(a, b, __fmul_rn(c, d)); }
-__device__ __forceinline__ float sum3(float a, float b, float c, float d, float e, float f) {
-    return __fmaf_rn(e, f, sum2(a, b, c, d));
-}
-using F3 = pg::V3<float>;
-__device__ __forceinline__ F3 f3(float4 v) { return pg::v3(v.x, v.y, v.z); }
+__device__ __forceinline__ float fma_t(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_t(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float mul_t(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_t(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float add_t(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double add_t(double a, double b) { return __dadd_rn(a, b); }
+template <class T>
+__device__ __forceinline__ T sum2(T a, T b, T c, T d) { return fma_t(a, b, mul_t(c, d)); }
+template <class T>
+__device__ __forceinline__ T sum3(T a, T b, T c, T d, T e, T f) { return fma_t(e, f, sum2(a, b, c, d)); }
+template <class T>
+__device__ __forceinline__ pg::V3<T> v3(const Vec4<T>& v) { return pg::v3(v.x, v.y, v.z); }
 
-__device__ __forceinline__ F3 obj_wind(const ObjConst& c, F3 p, float t, F3 vel) {
-    const float s = c.phase;
-    auto arg = [&](float a, float x, float b, float cc) { return sum3(a, x, b, t, cc, s); };
-    const float a1 = arg(0.9f, p.x, 1.3f, 1.0f), a2 = arg(2.3f, p.z, 2.1f, 1.7f), a3 = arg(4.1f, p.y, 3.3f, 0.4f);
-    const float b1 = arg(1.1f, p.x, 1.7f, 2.2f), b2 = arg(3.1f, p.z, 2.9f, 0.9f);
-    const float c1 = arg(1.4f, p.x, 2.3f, 3.1f), c2 = arg(2.7f, p.y, 1.9f, 1.2f);
-    const float gx = sum3(0.55f, pg::p_sin(a1), 0.35f, pg::p_sin(a2), 0.25f, pg::p_sin(a3));
-    const float gy = sum2(0.50f, pg::p_sin(b1), 0.30f, pg::p_sin(b2));
-    const float gz = sum2(0.30f, pg::p_sin(c1), 0.20f, pg::p_sin(c2));
-    const float G = c.gust;
-    const float wx = __fmaf_rn(G, gx, c.base_x);
-    const float wy = __fmaf_rn(G, gy, c.base_y);
-    return pg::v3(__fadd_rn(vel.x, -wx), __fadd_rn(vel.y, -wy), __fmaf_rn(-G, gz, vel.z));
+template <class T>
+__device__ __forceinline__ pg::V3<T> obj_wind(const ObjConst<T>& c, pg::V3<T> p, T t, pg::V3<T> vel) {
+    const T s = c.phase;
+    auto arg = [&](T a, T x, T b, T cc) { return sum3(a, x, b, t, cc, s); };
+    const T a1 = arg(T(0.9f), p.x, T(1.3f), T(1.0f)), a2 = arg(T(2.3f), p.z, T(2.1f), T(1.7f)), a3 = arg(T(4.1f), p.y, T(3.3f), T(0.4f));
+    const T b1 = arg(T(1.1f), p.x, T(1.7f), T(2.2f)), b2 = arg(T(3.1f), p.z, T(2.9f), T(0.9f));
+    const T c1 = arg(T(1.4f), p.x, T(2.3f), T(3.1f)), c2 = arg(T(2.7f), p.y, T(1.9f), T(1.2f));
+    const T gx = sum3(T(0.55f), pg::p_sin(a1), T(0.35f), pg::p_sin(a2), T(0.25f), pg::p_sin(a3));
+    const T gy = sum2(T(0.50f), pg::p_sin(b1), T(0.30f), pg::p_sin(b2));
+    const T gz = sum2(T(0.30f), pg::p_sin(c1), T(0.20f), pg::p_sin(c2));
+    const T G = c.gust;
+    const T wx = fma_t(G, gx, c.base_x);
+    const T wy = fma_t(G, gy, c.base_y);
+    return pg::v3(add_t(vel.x, -wx), add_t(vel.y, -wy), fma_t(-G, gz, vel.z));
 }
 
-__device__ __forceinline__ void obj_publish_rotation(ObjBlock& b, int m, int par, bool write, const float (&q)[4], F3 w, float cf) {
-    const float qw = q[0], x = q[1], y = q[2], z = q[3];
-    const float yy = __fmul_rn(y, y), zz = __fmul_rn(z, z);
-    const float r00 = __fmaf_rn(-2.f, __fadd_rn(yy, zz), 1.f), r11 = __fmaf_rn(-2.f, __fmaf_rn(x, x, zz), 1.f);
-    const float r22 = __fmaf_rn(-2.f, __fmaf_rn(x, x, yy), 1.f);
-    const float r01 = 2.f * sum2(x, y, -qw, z), r02 = 2.f * sum2(qw, y, x, z), r10 = 2.f * sum2(x, y, qw, z);
-    const float r12 = 2.f * sum2(y, z, -qw, x), r20 = 2.f * sum2(-qw, y, x, z), r21 = 2.f * sum2(y, z, qw, x);
+template <class T>
+__device__ __forceinline__ void obj_publish_rotation(ObjBlock<T>& b, int m, int par, bool write, const T (&q)[4], pg::V3<T> w, T cf) {
+    const T qw = q[0], x = q[1], y = q[2], z = q[3];
+    const T yy = mul_t(y, y), zz = mul_t(z, z);
+    const T r00 = fma_t(T(-2), add_t(yy, zz), T(1)), r11 = fma_t(T(-2), fma_t(x, x, zz), T(1));
+    const T r22 = fma_t(T(-2), fma_t(x, x, yy), T(1));
+    const T r01 = T(2) * sum2(x, y, -qw, z), r02 = T(2) * sum2(qw, y, x, z), r10 = T(2) * sum2(x, y, qw, z);
+    const T r12 = T(2) * sum2(y, z, -qw, x), r20 = T(2) * sum2(-qw, y, x, z), r21 = T(2) * sum2(y, z, qw, x);
     if (!write) return;
-    b.q[m] = make_float4(qw, x, y, z);
-    b.w[m] = make_float4(w.x, w.y, w.z, 0.f);
-    b.rows[par][m][0] = make_float4(r00, r01, r02, r10);
-    b.rows[par][m][1] = make_float4(r11, r12, r20, r21);
-    b.rows[par][m][2] = make_float4(r22, 0.f, 0.f, cf);
+    using V4 = Vec4<T>;
+    b.q[m] = V4{qw, x, y, z};
+    b.w[m] = V4{w.x, w.y, w.z, T(0)};
+    b.rows[par][m][0] = V4{r00, r01, r02, r10};
+    b.rows[par][m][1] = V4{r11, r12, r20, r21};
+    b.rows[par][m][2] = V4{r22, T(0), T(0), cf};
 }
-__device__ __forceinline__ void obj_publish_translation(ObjBlock& b, int m, bool write, const ObjConst& c, F3 pos, F3 vel, float t, int step) {
-    const F3 va = obj_wind(c, pos, t, vel);
+template <class T>
+__device__ __forceinline__ void obj_publish_translation(ObjBlock<T>& b, int m, bool write, const ObjConst<T>& c, pg::V3<T> pos, pg::V3<T> vel, T t, int step) {
+    const pg::V3<T> va = obj_wind(c, pos, t, vel);
     if (!write) return;
-    b.pos_t[m] = make_float4(pos.x, pos.y, pos.z, t);
-    b.vel[m] = make_float4(vel.x, vel.y, vel.z, 0.f);
+    using V4 = Vec4<T>;
+    b.pos_t[m] = V4{pos.x, pos.y, pos.z, t};
+    b.vel[m] = V4{vel.x, vel.y, vel.z, T(0)};
     b.step[m] = step;
-    b.va[m] = make_float4(va.x, va.y, va.z, 0.f);
+    b.va[m] = V4{va.x, va.y, va.z, T(0)};
 }
 
-__device__ __forceinline__ F3 obj_sum(const ObjBlock& b, int m, int k) {
-    F3 t = f3(b.part[m][k]);
+template <class T>
+__device__ __forceinline__ pg::V3<T> obj_sum(const ObjBlock<T>& b, int m, int k) {
+    pg::V3<T> t = v3(b.part[m][k]);
 #pragma unroll
-    for (int w = 1; w < kObjW; w++) t = t + f3(b.part[m][2 * w + k]);
+    for (int w = 1; w < kObjW; w++) t = t + v3(b.part[m][2 * w + k]);
     return t;
 }
 
-__global__ void __launch_bounds__(32 * kObjW, 5) k_obj_flights(ObjArgs a) {
+template <class T>
+__global__ void __launch_bounds__(32 * kObjW, sizeof(T) == 4 ? 5 : 2) k_obj_flights(ObjArgs a) {
+    using Block = ObjBlock<T>;
+    using V3T = pg::V3<T>;
+    using V4 = Vec4<T>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    ObjBlock& b = *reinterpret_cast<ObjBlock*>(smem_raw);
+    Block& b = *reinterpret_cast<Block*>(smem_raw);
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
     int lane;
     asm volatile("mov.u32 %0, %%laneid;" : "=r"(lane));
@@ -481,7 +366,7 @@ __global__ void __launch_bounds__(32 * kObjW, 5) k_obj_flights(ObjArgs a) {
                         break;
                     }
                     const int p = f / a.nseeds, si = f - p * a.nseeds;
-                    const float* pl = reinterpret_cast<const float*>(a.plane) + (size_t)p * kObjPlaneStride;
+                    const T* pl = reinterpret_cast<const T*>(a.plane) + (size_t)p * kObjPlaneStride;
                     const int nt = (int)pl[7];
                     if (nt <= 0) {  // does not fit the print volume
                         if (lane == 0) a.dist[f] = -100.0;
@@ -490,37 +375,37 @@ __global__ void __launch_bounds__(32 * kObjW, 5) k_obj_flights(ObjArgs a) {
                     const int seed = a.seeds[si] + (a.vary ? p * 7919 : 0);
                     Scenario S;
                     scenario_desc(seed, &S);
-                    float sc[kScenN];
+                    T sc[kScenN];
 #pragma unroll
-                    for (int k = 0; k < kScenN; k++) sc[k] = S.v[k];
-                    F3 cg;
-                    float sigma, beta[6], I[6];
+                    for (int k = 0; k < kScenN; k++) sc[k] = (T)S.v[k];
+                    V3T cg;
+                    T sigma, beta[6], I[6];
 #pragma unroll
                     for (int q = 0; q < 6; q++) I[q] = pl[1 + q];
-                    pg::FlightP<float> P;
+                    pg::FlightP<T> P;
                     pg::printed(sc, pl[0], I, P, &cg, &sigma, beta);
-                    P.phase = seed_phase(seed);
-                    const float* pc = pl + 8;
+                    P.phase = (T)seed_phase(seed);
+                    const T* pc = pl + 8;
                     for (int i = lane; i - lane < nt; i += 32) {
-                        F3 rb = pg::v3(0.f, 0.f, 0.f), nb = rb;
-                        float ak = 0.f;
+                        V3T rb = pg::v3(T(0), T(0), T(0)), nb = rb;
+                        T ak = T(0);
                         if (i < nt)
                             pg::stage(pg::v3(pc[i], pc[kNtMax + i], pc[2 * kNtMax + i]), pc[3 * kNtMax + i],
                                       pg::v3(pc[4 * kNtMax + i], pc[5 * kNtMax + i], pc[6 * kNtMax + i]), cg, sc[pg::SC_RHO],
                                       sc[pg::SC_WP], sc[pg::SC_WR], &rb, &nb, &ak);
-                        b.rb[warp][i] = make_float4(rb.x, rb.y, rb.z, ak);
-                        b.nxy[warp][i] = make_float2(nb.x, nb.y);
+                        b.rb[warp][i] = V4{rb.x, rb.y, rb.z, ak};
+                        b.nxy[warp][i] = Vec2<T>{nb.x, nb.y};
                         b.nz[warp][i] = nb.z;
                     }
-                    const pg::St<float> s = pg::release(sc, P, cg, (F3*)nullptr, (F3*)nullptr);
-                    ObjConst c;
+                    const pg::St<T> s = pg::release(sc, P, cg, (V3T*)nullptr, (V3T*)nullptr);
+                    ObjConst<T> c;
 #pragma unroll
                     for (int k = 0; k < 6; k++) c.I[k] = P.I[k];
 #pragma unroll
                     for (int k = 0; k < 9; k++) c.invI[k] = P.invI[k];
                     c.cf = P.cf; c.mass = P.mass; c.invmass = P.invmass; c.gust = P.gust; c.phase = P.phase;
-                    c.base_x = P.base_x; c.base_y = P.base_y; c.pad0 = c.pad1 = 0.f;
-                    const float4* o = reinterpret_cast<const float4*>(&c);
+                    c.base_x = P.base_x; c.base_y = P.base_y; c.pad0 = c.pad1 = T(0);
+                    const V4* o = reinterpret_cast<const V4*>(&c);
                     if (lane == 0) {
 #pragma unroll
                         for (int k = 0; k < 6; k++) b.cst[k][warp] = o[k];
@@ -535,25 +420,25 @@ __global__ void __launch_bounds__(32 * kObjW, 5) k_obj_flights(ObjArgs a) {
             __syncthreads();
         }
         if ((b.nt[0] | b.nt[1] | b.nt[2] | b.nt[3]) == 0) break;
-        float v[24];
+        T v[24];
 #pragma unroll
         for (int k = 0; k < kObjW; k++) {
-            float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            T acc[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
             const int nt = b.nt[k], i0 = 32 * ((warp - k) & 3);
             if (i0 < nt) {
-                const float4 m0 = b.rows[par][k][0], m1 = b.rows[par][k][1], m2 = b.rows[par][k][2], va = b.va[k];
-                pg::Pre<float> q;
+                const V4 m0 = b.rows[par][k][0], m1 = b.rows[par][k][1], m2 = b.rows[par][k][2], va = b.va[k];
+                pg::Pre<T> q;
                 q.vb = pg::v3(sum3(m0.x, va.x, m0.w, va.y, m1.z, va.z), sum3(m0.y, va.x, m1.x, va.y, m1.w, va.z),
                               sum3(m0.z, va.x, m1.y, va.y, m2.x, va.z));
-                q.w = f3(b.w[k]);
-                const float4* rb = b.rb[k] + i0 + lane;
-                const float2* nxy = b.nxy[k] + i0 + lane;
-                const float* nz = b.nz[k] + i0 + lane;
+                q.w = v3(b.w[k]);
+                const V4* rb = b.rb[k] + i0 + lane;
+                const Vec2<T>* nxy = b.nxy[k] + i0 + lane;
+                const T* nz = b.nz[k] + i0 + lane;
                 auto panel = [&](int o) {
-                    const float4 r = rb[o];
-                    const float2 n = nxy[o];
-                    F3 fo, tq;
-                    pg::panel_fwd(q, f3(r), pg::v3(n.x, n.y, nz[o]), r.w, m2.w, &fo, &tq);
+                    const V4 r = rb[o];
+                    const Vec2<T> n = nxy[o];
+                    V3T fo, tq;
+                    pg::panel_fwd(q, v3(r), pg::v3(n.x, n.y, nz[o]), r.w, m2.w, &fo, &tq);
                     acc[0] += fo.x; acc[1] += fo.y; acc[2] += fo.z;
                     acc[3] += tq.x; acc[4] += tq.y; acc[5] += tq.z;
                 };
@@ -566,53 +451,53 @@ __global__ void __launch_bounds__(32 * kObjW, 5) k_obj_flights(ObjArgs a) {
 #pragma unroll
             for (int c = 0; c < 6; c++) v[6 * k + c] = acc[c];
         }
-        const float total = warp_sum24(v, lane);
-        if ((lane & 3) != 3) reinterpret_cast<float*>(&b.part[m][2 * ((warp - m) & 3)])[lane & 7] = total;
+        const T total = warp_sum24(v, lane);
+        if ((lane & 3) != 3) reinterpret_cast<T*>(&b.part[m][2 * ((warp - m) & 3)])[lane & 7] = total;
         __syncthreads();
         if (warp == turn) {
-            ObjConst c;
-            float4* o = reinterpret_cast<float4*>(&c);
+            ObjConst<T> c;
+            V4* o = reinterpret_cast<V4*>(&c);
 #pragma unroll
             for (int k = 0; k < 4; k++) o[k] = b.cst[k][m];
-            const F3 Tb = obj_sum(b, m, 1), w = f3(b.w[m]);
-            const float4 q4 = b.q[m];
-            const F3 Iw = pg::v3(sum3(c.I[0], w.x, c.I[3], w.y, c.I[4], w.z), sum3(c.I[3], w.x, c.I[1], w.y, c.I[5], w.z),
+            const V3T Tb = obj_sum(b, m, 1), w = v3(b.w[m]);
+            const V4 q4 = b.q[m];
+            const V3T Iw = pg::v3(sum3(c.I[0], w.x, c.I[3], w.y, c.I[4], w.z), sum3(c.I[3], w.x, c.I[1], w.y, c.I[5], w.z),
                                  sum3(c.I[5], w.y, c.I[4], w.x, c.I[2], w.z));
-            const F3 gy = pg::v3(sum2(w.y, Iw.z, -w.z, Iw.y), sum2(w.z, Iw.x, -w.x, Iw.z), sum2(w.x, Iw.y, -w.y, Iw.x));
-            const F3 tq = Tb - gy;
-            const F3 dw = pg::v3(sum3(c.invI[0], tq.x, c.invI[1], tq.y, c.invI[2], tq.z), sum3(c.invI[3], tq.x, c.invI[4], tq.y, c.invI[5], tq.z),
+            const V3T gy = pg::v3(sum2(w.y, Iw.z, -w.z, Iw.y), sum2(w.z, Iw.x, -w.x, Iw.z), sum2(w.x, Iw.y, -w.y, Iw.x));
+            const V3T tq = Tb - gy;
+            const V3T dw = pg::v3(sum3(c.invI[0], tq.x, c.invI[1], tq.y, c.invI[2], tq.z), sum3(c.invI[3], tq.x, c.invI[4], tq.y, c.invI[5], tq.z),
                                  sum3(c.invI[6], tq.x, c.invI[7], tq.y, c.invI[8], tq.z));
-            const float dt = pg::kDt;
-            const F3 w1 = pg::v3(__fmaf_rn(dw.x, dt, w.x), __fmaf_rn(dw.y, dt, w.y), __fmaf_rn(dw.z, dt, w.z));
-            const F3 wn = pg::clamp_len(w1, 150.f);
-            const float q[4] = {q4.x, q4.y, q4.z, q4.w};
-            const float dq[4] = {-sum3(q[1], wn.x, q[2], wn.y, q[3], wn.z), __fmaf_rn(-q[3], wn.y, sum2(q[0], wn.x, q[2], wn.z)),
-                                 __fmaf_rn(q[3], wn.x, sum2(q[0], wn.y, -q[1], wn.z)), __fmaf_rn(-q[2], wn.x, sum2(q[0], wn.z, q[1], wn.y))};
-            const float h = 0.5f * dt;
-            float qn[4], l2 = 0.f;
+            const T dt = T(pg::kDt);
+            const V3T w1 = pg::v3(fma_t(dw.x, dt, w.x), fma_t(dw.y, dt, w.y), fma_t(dw.z, dt, w.z));
+            const V3T wn = pg::clamp_len(w1, T(150));
+            const T q[4] = {q4.x, q4.y, q4.z, q4.w};
+            const T dq[4] = {-sum3(q[1], wn.x, q[2], wn.y, q[3], wn.z), fma_t(-q[3], wn.y, sum2(q[0], wn.x, q[2], wn.z)),
+                                 fma_t(q[3], wn.x, sum2(q[0], wn.y, -q[1], wn.z)), fma_t(-q[2], wn.x, sum2(q[0], wn.z, q[1], wn.y))};
+            const T h = T(0.5) * dt;
+            T qn[4], l2 = T(0);
 #pragma unroll
-            for (int k = 0; k < 4; k++) { qn[k] = __fmaf_rn(h, dq[k], q[k]); l2 = k ? __fmaf_rn(qn[k], qn[k], l2) : __fmul_rn(qn[k], qn[k]); }
-            const float il = pg::p_rsqrt(l2);
-            const float qo[4] = {qn[0] * il, qn[1] * il, qn[2] * il, qn[3] * il};
+            for (int k = 0; k < 4; k++) { qn[k] = fma_t(h, dq[k], q[k]); l2 = k ? fma_t(qn[k], qn[k], l2) : mul_t(qn[k], qn[k]); }
+            const T il = pg::p_rsqrt(l2);
+            const T qo[4] = {qn[0] * il, qn[1] * il, qn[2] * il, qn[3] * il};
             __syncwarp();
             obj_publish_rotation(b, m, par ^ 1, leads, qo, wn, c.cf);
         } else if (warp == ((turn + 1) & 3)) {
-            ObjConst c;
-            float4* o = reinterpret_cast<float4*>(&c);
+            ObjConst<T> c;
+            V4* o = reinterpret_cast<V4*>(&c);
             o[4] = b.cst[4][m]; o[5] = b.cst[5][m];
-            const float4 m0 = b.rows[par][m][0], m1 = b.rows[par][m][1], m2 = b.rows[par][m][2], p4 = b.pos_t[m];
-            const F3 Fb = obj_sum(b, m, 0);
-            F3 Fw = pg::v3(sum3(m0.x, Fb.x, m0.y, Fb.y, m0.z, Fb.z), sum3(m0.w, Fb.x, m1.x, Fb.y, m1.y, Fb.z),
+            const V4 m0 = b.rows[par][m][0], m1 = b.rows[par][m][1], m2 = b.rows[par][m][2], p4 = b.pos_t[m];
+            const V3T Fb = obj_sum(b, m, 0);
+            V3T Fw = pg::v3(sum3(m0.x, Fb.x, m0.y, Fb.y, m0.z, Fb.z), sum3(m0.w, Fb.x, m1.x, Fb.y, m1.y, Fb.z),
                            sum3(m1.z, Fb.x, m1.w, Fb.y, m2.x, Fb.z));
-            Fw.z = __fmaf_rn(-c.mass, pg::kGrav, Fw.z);
-            const float dt = pg::kDt, kv = __fmul_rn(c.invmass, dt);
-            const F3 vel = f3(b.vel[m]);
-            const F3 vel1 = pg::v3(__fmaf_rn(Fw.x, kv, vel.x), __fmaf_rn(Fw.y, kv, vel.y), __fmaf_rn(Fw.z, kv, vel.z));
-            pg::St<float> before{}, after{};
-            before.pos = f3(p4);
-            after.vel = pg::clamp_len(vel1, 60.f);
-            after.pos = pg::v3(__fmaf_rn(after.vel.x, dt, before.pos.x), __fmaf_rn(after.vel.y, dt, before.pos.y), __fmaf_rn(after.vel.z, dt, before.pos.z));
-            float t = __fadd_rn(p4.w, dt), d = 0.f;
+            Fw.z = fma_t(-c.mass, T(pg::kGrav), Fw.z);
+            const T dt = T(pg::kDt), kv = mul_t(c.invmass, dt);
+            const V3T vel = v3(b.vel[m]);
+            const V3T vel1 = pg::v3(fma_t(Fw.x, kv, vel.x), fma_t(Fw.y, kv, vel.y), fma_t(Fw.z, kv, vel.z));
+            pg::St<T> before{}, after{};
+            before.pos = v3(p4);
+            after.vel = pg::clamp_len(vel1, T(60));
+            after.pos = pg::v3(fma_t(after.vel.x, dt, before.pos.x), fma_t(after.vel.y, dt, before.pos.y), fma_t(after.vel.z, dt, before.pos.z));
+            T t = add_t(p4.w, dt), d = T(0);
             int kind = 0;
             const int step = b.step[m];
             const bool live = b.nt[m] > 0;
@@ -622,7 +507,7 @@ __global__ void __launch_bounds__(32 * kObjW, 5) k_obj_flights(ObjArgs a) {
             if (ended) {
                 if (leads && live) { a.dist[flight] = (double)d; b.nt[m] = -1; }
             } else {
-                if ((step + 1) % kChunk == 0) t = (float)(step + 1) * (float)pg::kDt;
+                if ((step + 1) % kChunk == 0) t = T((double)(step + 1)) * T(pg::kDt);
                 obj_publish_translation(b, m, leads, c, after.pos, after.vel, t, step + 1);
             }
         }
@@ -640,26 +525,21 @@ __global__ void __launch_bounds__(32) k_obj_weights(ObjArgs a) {
     if (tid == 0) a.obj[p] = (double)pg::objective_weights(d, S, w);
 }
 
-template <class T>
-size_t forward_smem() {
-    return (size_t)(2 * kObjW * 8 + 2) * sizeof(T) + (size_t)7 * kNtMax * sizeof(T);
-}
+constexpr size_t kForwardSmem = (size_t)(2 * kObjW * 8 + 2) * sizeof(float) + (size_t)7 * kNtMax * sizeof(float);
 
 template <class T>
 cudaError_t launch_t(const ObjArgs& a, int nsm, cudaStream_t s) {
-    // FP32 by number of flights: milliseconds with a flight per block / four, 128 x 8 1.32 / 1.46, 256 x 8
-    // 1.99 / 2.01, 384 x 8 2.36 / 2.18, 512 x 8 2.99 / 2.24.  FP64 with a flight per block / four: 17.1 / 17.1
-    // at 16 x 2, 37.5 / 34.4 at 64 x 8, 162 / 93 at 512 x 8.
-    constexpr bool FP32 = sizeof(T) == 4;
-    const bool many = FP32 && (long long)a.pop * a.nseeds > 14LL * nsm;
-    const void* fn;
-    size_t smem;
-    if constexpr (FP32) {
-        fn = many ? (const void*)k_obj_flights : (const void*)k_obj_forward<T>;
-        smem = many ? sizeof(ObjBlock) : forward_smem<T>();
-    } else {
-        fn = (const void*)k_obj_forward4<T>;
-        smem = kObjW * sizeof(ObjSlot<T>);
+    // Milliseconds with a flight per block / four.  FP32: 128 x 8 1.32 / 1.46, 256 x 8 1.99 / 2.01, 384 x 8
+    // 2.36 / 2.18, 512 x 8 2.99 / 2.24.  FP64: 1 x 1 4.9 / 3.7, 20 x 8 26.6 / 23.9, 512 x 8 160 / 72.
+    const void* fn = (const void*)k_obj_flights<T>;
+    size_t smem = sizeof(ObjBlock<T>);
+    bool single = false;
+    if constexpr (sizeof(T) == 4) {
+        single = (long long)a.pop * a.nseeds <= 14LL * nsm;
+        if (single) {
+            fn = (const void*)k_obj_forward;
+            smem = kForwardSmem;
+        }
     }
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -670,12 +550,8 @@ cudaError_t launch_t(const ObjArgs& a, int nsm, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     const int grid = (bpsm > 0 ? bpsm : 1) * nsm;
     k_obj_prepare<T><<<a.pop, kObjThreads, 0, s>>>(a);
-    if constexpr (FP32) {
-        if (many) k_obj_flights<<<grid, 32 * kObjW, smem, s>>>(a);
-        else k_obj_forward<T><<<grid, 32 * kObjW, smem, s>>>(a);
-    } else {
-        k_obj_forward4<T><<<grid, 32 * kObjW, smem, s>>>(a);
-    }
+    if (single) k_obj_forward<<<grid, 32 * kObjW, smem, s>>>(a);
+    else k_obj_flights<T><<<grid, 32 * kObjW, smem, s>>>(a);
     if (a.obj) k_obj_weights<T><<<a.pop, 32, 0, s>>>(a);
     return cudaGetLastError();
 }
