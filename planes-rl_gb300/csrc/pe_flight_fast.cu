@@ -34,12 +34,13 @@ __device__ __forceinline__ void rec_fill(const FlightArgs& a, int flight, int fr
 // CAP = 3 launches one-warp blocks, 11 per SM (registers <= 184, no spills): at 16 lanes that is
 // all the 2-flight slots shared memory holds (11 x (2 x 9,856 B + 1 KB reserved) of 228 KB), one
 // warp more per SM than the uncapped kernel's 198 registers leave room for.
-// With 32 lanes and FlightArgs.landed a flight of the launch's last few is left to pe_flight_wide.cu.
+// HAND = true leaves the flights of the launch's last few to pe_flight_wide.cu (FlightArgs.landed), asked for
+// every 16 steps outside the loop of the steps: inside it, even never taken, it cost 4 % of a 2,048 x 8 run.
 // REC = true adds the reference's pose recording and launch grid (pe_sim only).
 // GRAD = true is pe_grad's forward pass: every flight from its set-up record (FlightArgs.grad_setup),
 // smoothed distances, and per flight its checkpoints, every step's body force and torque and how it
 // ended (FlightArgs.grad_*); one launch over all flights.
-template <int LPF, int CAP, bool REC = false, bool GRAD = false>
+template <int LPF, int CAP, bool REC = false, bool GRAD = false, bool HAND = false>
 __global__ void __launch_bounds__(CAP == 3 ? 32 : (CAP ? 128 : 256), CAP == 1 ? 5 : (CAP == 2 ? 4 : (CAP == 3 ? 11 : 1)))
     k_flight_fast(FlightArgs a) {
     extern __shared__ float4 smem[];
@@ -69,7 +70,7 @@ __global__ void __launch_bounds__(CAP == 3 ? 32 : (CAP ? 128 : 256), CAP == 1 ? 
                     a.dist[flight] = -100.0f;
                     a.steps[flight] = 0;
                     a.grad_kind[flight] = 0;
-                    if (LPF == 32 && a.landed) atomicAdd(a.landed, 1);
+                    if (HAND) atomicAdd(a.landed, 1);
                 }
                 continue;
             }
@@ -89,7 +90,7 @@ __global__ void __launch_bounds__(CAP == 3 ? 32 : (CAP ? 128 : 256), CAP == 1 ? 
                     if (j == 0) {
                         a.dist[flight] = -100.0f;
                         a.steps[flight] = 0;
-                        if (LPF == 32 && !REC && a.landed) atomicAdd(a.landed, 1);
+                        if (HAND) atomicAdd(a.landed, 1);
                     }
                     if (REC && a.rec) rec_fill(a, flight, -1, st, j, LPF);
                     continue;
@@ -115,40 +116,42 @@ __global__ void __launch_bounds__(CAP == 3 ? 32 : (CAP ? 128 : 256), CAP == 1 ? 
         so.kind = 0;
         int to_ck = GRAD ? a.grad_K : 0, ck_i = 0;  // steps to the next checkpoint, its index
         int seen = 0;                               // flights of the launch that had ended 16 steps ago
-        bool give = false;
-        for (; step < end; step++) {
-            if (LPF == 32 && !REC && a.landed && (step & 15) == 0) {  // few left: pe_flight_wide.cu takes them
-                give = n_work - __shfl_sync(mask, seen, 0) <= a.hand_over;
-                if (give) break;
+        while (step < end && !done) {
+            int stop = end;
+            if (HAND) {
+                if (n_work - __shfl_sync(mask, seen, 0) <= a.hand_over) break;
                 seen = *(volatile int*)a.landed;
+                stop = min(end, (step | 15) + 1);
             }
-            if (REC && a.rec && j == 0 && step % a.rec_every == 0) rec_put(a, flight, step, st, 1.f);
-            done = fast_step<LPF>(fc, pp, nt, j, mask, st, step, a.max_steps, GRAD ? 1 : a.smooth, &fit, nullptr,
-                                  GRAD ? &so : nullptr);
-            if (GRAD && j == 0) {
-                if (fsum) {
-                    float4* d4 = reinterpret_cast<float4*>(fsum + (size_t)step * 8);
-                    d4[0] = make_float4(so.fb[0], so.fb[1], so.fb[2], so.fb[3]);
-                    d4[1] = make_float4(so.fb[4], so.fb[5], 0.0f, 0.0f);
+            for (; step < stop; step++) {
+                if (REC && a.rec && j == 0 && step % a.rec_every == 0) rec_put(a, flight, step, st, 1.f);
+                done = fast_step<LPF>(fc, pp, nt, j, mask, st, step, a.max_steps, GRAD ? 1 : a.smooth, &fit, nullptr,
+                                      GRAD ? &so : nullptr);
+                if (GRAD && j == 0) {
+                    if (fsum) {
+                        float4* d4 = reinterpret_cast<float4*>(fsum + (size_t)step * 8);
+                        d4[0] = make_float4(so.fb[0], so.fb[1], so.fb[2], so.fb[3]);
+                        d4[1] = make_float4(so.fb[4], so.fb[5], 0.0f, 0.0f);
+                    }
                 }
-            }
-            if (GRAD && --to_ck == 0) {  // after step + 1 = (ck_i + 1) * K steps
-                to_ck = a.grad_K;
-                ++ck_i;
-                if (!done && j == 0) {
-                    FlightState c = st;  // as the next step starts: the clock restarts every 600 steps
-                    if ((step + 1) % kChunk == 0) c.t = mul_((float)(step + 1), PE_DT);
-                    *reinterpret_cast<FlightState*>(ck + (size_t)ck_i * 16) = c;
+                if (GRAD && --to_ck == 0) {  // after step + 1 = (ck_i + 1) * K steps
+                    to_ck = a.grad_K;
+                    ++ck_i;
+                    if (!done && j == 0) {
+                        FlightState c = st;  // as the next step starts: the clock restarts every 600 steps
+                        if ((step + 1) % kChunk == 0) c.t = mul_((float)(step + 1), PE_DT);
+                        *reinterpret_cast<FlightState*>(ck + (size_t)ck_i * 16) = c;
+                    }
                 }
+                if (done) break;
             }
-            if (done) break;
         }
         if (done) {
             if (GRAD && j == 0) a.grad_kind[flight] = so.kind;
             if (j == 0) {
                 a.dist[flight] = fit;
                 a.steps[flight] = step + 1;
-                if (LPF == 32 && !REC && a.landed) atomicAdd(a.landed, 1);
+                if (HAND) atomicAdd(a.landed, 1);
             }
             if (REC && a.rec) {
                 __syncwarp(mask);  // lane 0's alive frames precede the frozen ones that may share a slot
@@ -243,6 +246,12 @@ cudaError_t launch_flight_fast(const FlightArgs& a, const FlightShape& sh, int g
                                  (int)smem);
         if (e != cudaSuccess) return e;
         k_flight_fast<16, 0, true><<<grid, threads, smem, s>>>(a);
+    } else if (a.landed) {  // the engine's own choice for middling batches
+        if (sh.lanes != 32 || sh.cap) return cudaErrorInvalidValue;
+        e = cudaFuncSetAttribute((const void*)&k_flight_fast<32, 0, false, false, true>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        k_flight_fast<32, 0, false, false, true><<<grid, threads, smem, s>>>(a);
     } else if (sh.lanes == 16) {
         launch_lanes<16>(a, sh.cap, grid, threads, smem, s);
     } else if (sh.lanes == 32) {
@@ -254,7 +263,7 @@ cudaError_t launch_flight_fast(const FlightArgs& a, const FlightShape& sh, int g
 }
 
 cudaError_t grad_forward_configure(int bps[2]) {
-    const void* fn[2] = {(const void*)&k_flight_fast<32, 0, false, true>, (const void*)&k_flight_fast<16, 3, false, true>};
+    const void* fn[2] = {(const void*)&k_flight_fast<32, 0, false, true, true>, (const void*)&k_flight_fast<16, 3, false, true>};
     const int threads[2] = {128, 32};
     const size_t smem[2] = {4 * paired_bytes<32>(), 2 * paired_bytes<16>()};
     for (int i = 0; i < 2; i++) {
@@ -283,7 +292,7 @@ cudaError_t launch_grad_forward(const FlightArgs& a, int nsm, const int bps[2], 
         return cudaGetLastError();
     }
     if (!a.landed || !a.active_out || !a.n_active_out || !wide_work) return cudaErrorInvalidValue;
-    k_flight_fast<32, 0, false, true><<<bps[0] * nsm, 128, 4 * paired_bytes<32>(), s>>>(a);
+    k_flight_fast<32, 0, false, true, true><<<bps[0] * nsm, 128, 4 * paired_bytes<32>(), s>>>(a);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     w.active_in = a.active_out;

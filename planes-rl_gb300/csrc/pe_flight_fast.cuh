@@ -399,12 +399,26 @@ __device__ __forceinline__ vec3 fast_gyro(const FastConst& fc, vec3 w) {
                         fma_(fc.I[2], w.z, fma_(fc.I[5], w.y, mul_(fc.I[4], w.x))));
     return mk3(fma_(w.y, Iw.z, -mul_(w.z, Iw.y)), fma_(w.z, Iw.x, -mul_(w.x, Iw.z)), fma_(w.x, Iw.y, -mul_(w.y, Iw.x)));
 }
+// LATE: the limit on the rates is asked for after the attitude, so that a lone chain does not wait for the
+// branch (3 % of a step of pe_flight_wide.cu; kernels that others' warps keep busy lose 4 % by it).
+// A squared length safely below the limit's needs no root (a NaN takes the long way).
+__device__ __forceinline__ bool fast_limit(vec3& v, float safe, float limit) {
+    const float v2 = dot_(v, v);
+    if (v2 < safe) return false;
+    const float l = sqrtf(v2);
+    if (!(l > limit)) return false;
+    const float k = __fdiv_rn(limit, l);
+    v = mk3(mul_(v.x, k), mul_(v.y, k), mul_(v.z, k));
+    return true;
+}
+template <bool LATE = false>
 __device__ __forceinline__ void fast_rotate(const FastConst& fc, vec3 gyro, vec3 tb, vec3& w, quat4& q) {
     const vec3 tq = mk3(sub_(tb.x, gyro.x), sub_(tb.y, gyro.y), sub_(tb.z, gyro.z));
     const vec3 dw = mk3(fma_(fc.invI[2], tq.z, fma_(fc.invI[1], tq.y, mul_(fc.invI[0], tq.x))),
                         fma_(fc.invI[5], tq.z, fma_(fc.invI[4], tq.y, mul_(fc.invI[3], tq.x))),
                         fma_(fc.invI[8], tq.z, fma_(fc.invI[7], tq.y, mul_(fc.invI[6], tq.x))));
     w = mk3(fma_(dw.x, PE_DT, w.x), fma_(dw.y, PE_DT, w.y), fma_(dw.z, PE_DT, w.z));
+    if (!LATE) fast_limit(w, 22499.f, 150.f);
     // q += 0.5 dt q (0, w); normalize
     auto turn = [&](vec3 v) {
         const float h = mul_(0.5f, PE_DT);
@@ -417,36 +431,20 @@ __device__ __forceinline__ void fast_rotate(const FastConst& fc, vec3 gyro, vec3
         return mkq(mul_(qn.w, il), mul_(qn.x, il), mul_(qn.y, il), mul_(qn.z, il));
     };
     quat4 next = turn(w);
-    // A squared length safely below the limit's needs no root (a NaN takes the long way).  Asked after the
-    // attitude, so that the chain does not wait for the branch.
-    const float w2 = dot_(w, w);
-    if (!(w2 < 22499.f)) {
-        const float wl = sqrtf(w2);
-        if (wl > 150.f) {
-            const float k = __fdiv_rn(150.f, wl);
-            w = mk3(mul_(w.x, k), mul_(w.y, k), mul_(w.z, k));
-            next = turn(w);
-        }
-    }
+    if (LATE && fast_limit(w, 22499.f, 150.f)) next = turn(w);
     q = next;
 }
 // The integrator's translation from the world-frame aerodynamic force Fs.
+template <bool LATE = false>
 __device__ __forceinline__ void fast_translate(const FastConst& fc, vec3 Fs, vec3& vel, vec3& pos) {
     Fs.z = fma_(-fc.mass, PE_GRAV, Fs.z);
     const float kv = mul_(fc.invmass, PE_DT);
     vel = mk3(fma_(Fs.x, kv, vel.x), fma_(Fs.y, kv, vel.y), fma_(Fs.z, kv, vel.z));
-    const float v2 = dot_(vel, vel);
+    if (!LATE) fast_limit(vel, 3599.f, 60.f);
     const vec3 from = pos;
     auto move = [&]() { pos = mk3(fma_(vel.x, PE_DT, from.x), fma_(vel.y, PE_DT, from.y), fma_(vel.z, PE_DT, from.z)); };
     move();
-    if (!(v2 < 3599.f)) {
-        const float vl = sqrtf(v2);
-        if (vl > 60.f) {
-            const float k = __fdiv_rn(60.f, vl);
-            vel = mk3(mul_(vel.x, k), mul_(vel.y, k), mul_(vel.z, k));
-            move();
-        }
-    }
+    if (LATE && fast_limit(vel, 3599.f, 60.f)) move();
 }
 // Whether the flight ends at `step`.
 __device__ __forceinline__ bool fast_over(vec3 pos, vec3 vel, int step, int max_steps) {

@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(32 * kWideWarps, 4) k_flight_wide(FlightArgs a
                 if constexpr (w == 0) {
                     const vec3 gyro = fast_gyro(fc, st.wb);
                     block_sync();
-                    fast_rotate(fc, gyro, wide_fold(sm, 3, lane), st.wb, st.q);
+                    fast_rotate<true>(fc, gyro, wide_fold(sm, 3, lane), st.wb, st.q);
                     vec3 n0, n1, n2;
                     fast_rows(st.q, &n0, &n1, &n2);
                     wide_put_rot(sm, lane, n0, n1, n2, st.wb);
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(32 * kWideWarps, 4) k_flight_wide(FlightArgs a
                     before = st.pos;
                     block_sync();
                     const vec3 Fb = wide_fold(sm, 0, lane);
-                    fast_translate(fc, mk3(dot_(r0, Fb), dot_(r1, Fb), dot_(r2, Fb)), st.vel, st.pos);
+                    fast_translate<true>(fc, mk3(dot_(r0, Fb), dot_(r1, Fb), dot_(r2, Fb)), st.vel, st.pos);
                     const vec3 wind = wind_lanes(st.pos, tt, wind_of, fc.gust, fc.base_x, fc.base_y);
                     const int now = fast_over(st.pos, st.vel, step, a.max_steps) ? 1 : (step + 1 >= end ? 2 : 0);
                     sm.air = make_float4(sub_(st.vel.x, wind.x), sub_(st.vel.y, wind.y), sub_(st.vel.z, wind.z),
