@@ -793,7 +793,7 @@ def run_gpu(args, world, rank, local, pg):
         "nominal_plane_seconds_per_step": (pop * S + K * len(hseeds)) * args.max_steps / 600.0,
         "roofline": {"bound": "fp32", "kernel": "k_flight", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                      "frac": achieved / peak, "traffic": traffic,
-                     "traffic_source": "profiles/k_flight_fast_pop16k_x12.md, scaled per flight to the main launch",
+                     "traffic_source": "profiles/k_flight_quad_pop16k_x12.md, scaled per flight to the main launch",
                      "peak_source": "measured FP32 FMA probe (pe_fp32_peak_probe), same process",
                      "flop_per_panel_step": FLOP_PER_PANEL_STEP, "flop_per_step": FLOP_PER_STEP,
                      "flop_source": "the reference step's per-plane-step count (128 nt + 300, FMA = 2)",
