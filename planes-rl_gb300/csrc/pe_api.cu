@@ -2,9 +2,10 @@
 // replay, autotuner, the reference-compatible panelbuf layer and the parity probes.
 //
 // One evaluation is, on one stream:
-//   prepare (3 kernels) -> memset of the launch counters -> ceil(max_steps / chunk) flight
-//   launches (persistent grid; each reads the previous launch's list of airborne flights) ->
-//   scores.  With use_graph the whole sequence is captured once per shape and replayed.
+//   prepare (2 or 3 kernels) -> memset of the launch counters -> the flights -> scores.
+// The flights are the engine's own choice of one or two kernels (enqueue_fly_default), or in an explicit
+// shape ceil(max_steps / chunk) launches (persistent grid; each reads the previous launch's list of airborne
+// flights).  With use_graph the whole sequence is captured once per shape and replayed.
 #include <stdarg.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -91,7 +92,7 @@ bool valid_config(const pe_config& c) {
     return (c.lanes == 16 || c.lanes == 32) && c.warps >= 1 && c.warps <= 8 && c.chunk >= 1 &&
            c.chunk <= kMaxSteps && c.blocks >= 0 && (c.warps * 32) % c.lanes == 0 &&
            (c.formulation == 0 || c.formulation == 1) && (c.use_graph == 0 || c.use_graph == 1) &&
-           !(c.formulation == 0 && c.lanes != 32) &&  // the reference arithmetic runs one flight per warp
+           !(c.formulation == 0 && c.lanes != 32) &&  // the reference arithmetic sums in 32 lanes
            (c.reg_cap == 0 || ((c.reg_cap == 1 || c.reg_cap == 2) && c.formulation == 1 && c.warps <= 4) ||
             (c.reg_cap == 3 && c.formulation == 1 && c.warps == 1));
 }

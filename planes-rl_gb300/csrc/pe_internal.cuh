@@ -54,7 +54,7 @@ struct FlightArgs {
     int* active_out;        // flights still airborne after this launch (nullptr: last launch)
     int* n_active_out;
     int* work;              // fetch counter, zero at launch
-    // pe_flight_quad.cu only: flights of the launch that have ended; once no more than hand_over are left
+    // pe_flight_quad.cu and the hand-over of pe_flight_fast.cu: flights of the launch that have ended; once no more than hand_over are left
     // a warp leaves its own to active_out (nullptr: never)
     int* landed;
     int hand_over;
