@@ -2,7 +2,7 @@
 // replay, autotuner, the reference-compatible panelbuf layer and the parity probes.
 //
 // One evaluation is, on one stream:
-//   prepare (2 or 3 kernels) -> memset of the launch counters -> the flights -> scores.
+//   prepare (1 or 3 kernels) -> memset of the launch counters -> the flights -> scores.
 // The flights are the engine's own choice of one or two kernels (enqueue_fly_default), or in an explicit
 // shape ceil(max_steps / chunk) launches (persistent grid; each reads the previous launch's list of airborne
 // flights).  With use_graph the whole sequence is captured once per shape and replayed.

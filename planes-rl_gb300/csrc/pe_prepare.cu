@@ -1,6 +1,6 @@
 // pe_prepare.cu -- genome -> mesh -> mass properties -> packed panels (src/sim.cu:25-49).
 //
-// Three launches, two for at most kScanAlone genomes:
+// Three launches, k_mesh alone for at most kScanAlone genomes (each block counts the planes before its own):
 //   k_topo_scan   triangle count of each genome from its topology genes alone, block-local
 //                 exclusive scan, block totals out.
 //   k_scan_tot    exclusive scan of the block totals (one block, 1024 at a time); also the
@@ -14,7 +14,7 @@
 
 namespace pe {
 
-__global__ void __launch_bounds__(kScanBlock) k_topo_scan(PrepArgs a, int* total) {
+__global__ void __launch_bounds__(kScanBlock) k_topo_scan(PrepArgs a) {
     __shared__ int warp_tot[kScanBlock / 32];
     int p = blockIdx.x * kScanBlock + threadIdx.x;
     int n = 0;
@@ -42,10 +42,7 @@ __global__ void __launch_bounds__(kScanBlock) k_topo_scan(PrepArgs a, int* total
     __syncthreads();
     int excl = x - n + (w > 0 ? warp_tot[w - 1] : 0);
     if (p < a.pop) a.pt.off[p] = excl;  // block-local for now
-    if (threadIdx.x == kScanBlock - 1) {
-        a.block_sum[blockIdx.x] = total ? 0 : excl + n;
-        if (total) *total = excl + n;  // the only block: its totals need no scan of their own
-    }
+    if (threadIdx.x == kScanBlock - 1) a.block_sum[blockIdx.x] = excl + n;
 }
 
 // Exclusive scan of nblocks block totals in place, in tiles of 1024 with the running sum of the
@@ -89,24 +86,36 @@ __global__ void __launch_bounds__(1024) k_scan_tot(int* block_sum, int nblocks, 
 // A block per plane: all threads take the vertices and the sums' terms; then warp 0 adds in order while
 // warp 1 finds the extent, and once more while the others write the panels.  Bound by the two chains of
 // ordered sums and what leads up to them.  The preparation's launches together, with a warp per plane (two
-// per block of 46 KB, eight per SM) and so: 21.5 -> 17.5 us for one plane, 31 -> 23 for 8 to 128, 88 -> 69 for
-// 3,001, 184 -> 141 for 8,192, 1,920 -> 1,430 for 100,000.
+// per block of 46 KB, eight per SM) and so: 21.5 -> 17.5 us for one plane, 31 -> 23 for 8 to 128 (14.3 and 19.3
+// without the counting launch), 88 -> 69 for 3,001, 184 -> 141 for 8,192, 1,920 -> 1,430 for 100,000.
 constexpr int kMeshThreads = 128;
 
-__global__ void __launch_bounds__(kMeshThreads, 8) k_mesh(PrepArgs a) {
+// A small batch's preparation is its launches: 3.6 us of 18 at one genome, 5 of 24 at 128, for counting the
+// planes' triangles; a block's own count of the planes before it takes a thread each.
+constexpr int kScanAlone = kMeshThreads;
+
+template <bool ALONE>
+__global__ void __launch_bounds__(kMeshThreads, 8) k_mesh(PrepArgs a, int* total) {
     __shared__ float s_g[kGenomeN + 1];
     __shared__ vec3 s_v[kNvMax];
     __shared__ float s_com[5];
     __shared__ float s_terms[kMpTerms * kNtMax];
-    __shared__ int s_nt;
+    __shared__ int s_nt, s_before[kMeshThreads / 32];
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     const int p = blockIdx.x;
     if (tid < kGenomeN) s_g[tid] = a.genomes[(size_t)p * kGenomeN + tid];
+    if (ALONE) {  // triangles of the planes before this one, a thread each
+        const int n = tid < p ? topology(GenomeRef{a.genomes + (size_t)tid * kGenomeN}).nt : 0;
+        const int sum = __reduce_add_sync(0xffffffffu, n);
+        if (lane == 0) s_before[w] = sum;
+    }
     __syncthreads();
     GenomeRef g{s_g};
     const Topo tp = topology(g);
     for (int i = tid; i < tp.nv; i += kMeshThreads) s_v[i] = mesh_vertex(g, tp, i);
-    const int off = a.pt.off[p] + a.block_sum[p / kScanBlock];
+    const int off = ALONE ? s_before[0] + s_before[1] + s_before[2] + s_before[3]
+                          : a.pt.off[p] + a.block_sum[p / kScanBlock];
+    if (ALONE && tid == 0 && p == a.pop - 1) *total = off + tp.nt;
     __syncthreads();
     mass_first(s_v, tp, tid, kMeshThreads, s_terms);
     __syncthreads();
@@ -172,18 +181,16 @@ cudaError_t set_station_mode(int ieee) {
     return cudaMemcpyToSymbol(c_station_ieee, &v, sizeof(int));
 }
 
-// A small batch's preparation is its launches: without the scan's, 2 of 19 us at one genome; from some
-// hundreds on k_mesh and the flights hide it.
-constexpr int kScanAlone = 128;
-static_assert(kScanAlone <= kScanBlock, "one block counts them");
-
 int launch_prepare(const PrepArgs& a, int* d_total, cudaStream_t s) {
     int nb = (a.pop + kScanBlock - 1) / kScanBlock;
-    const bool alone = a.pop <= kScanAlone;
-    k_topo_scan<<<nb, kScanBlock, 0, s>>>(a, alone ? d_total : nullptr);
-    if (!alone) k_scan_tot<<<1, 1024, 0, s>>>(a.block_sum, nb, d_total);
-    k_mesh<<<a.pop, kMeshThreads, 0, s>>>(a);
-    return alone ? 2 : 3;
+    if (a.pop <= kScanAlone) {
+        k_mesh<true><<<a.pop, kMeshThreads, 0, s>>>(a, d_total);
+        return 1;
+    }
+    k_topo_scan<<<nb, kScanBlock, 0, s>>>(a);
+    k_scan_tot<<<1, 1024, 0, s>>>(a.block_sum, nb, d_total);
+    k_mesh<false><<<a.pop, kMeshThreads, 0, s>>>(a, d_total);
+    return 3;
 }
 
 }  // namespace pe

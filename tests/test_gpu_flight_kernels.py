@@ -180,3 +180,27 @@ def test_host_results(cuda, pe, oracle, pop, S, want):
         for k, v in out.items():
             assert np.array_equal(v, ref[k].cpu().numpy())
     e.close()
+
+
+@pytest.mark.parametrize("pop", [1, 2, 31, 33, 127, 128, 129, 300])
+def test_panel_offsets(cuda, pe, oracle, pop):
+    """Panel offsets counted by the mesh's own blocks (at most 128 planes) and by the scan: the exclusive
+    prefix of the topology's triangle counts, and the planes' panels as those of a plane alone."""
+    torch = cuda
+    G = oracle.grand(61, pop)
+
+    def table(g):
+        e, n = pe.Engine(0), g.shape[0]
+        e.eval_batch(torch.from_numpy(g).cuda(), n, [1], 0, 1, torch.empty(n, device="cuda"))
+        off, nt = (torch.empty(n, dtype=torch.int32, device="cuda") for _ in range(2))
+        ext, pc = torch.empty(n, 4, device="cuda"), torch.zeros(n * 344, 4, device="cuda")
+        total = e.plane_table(n, d_off=off, d_nt=nt, d_ext=ext, d_pc=pc)
+        torch.cuda.synchronize()
+        e.close()
+        return off.cpu().numpy(), nt.cpu().numpy(), ext[:, 3].cpu().numpy().astype(int), pc.cpu().numpy(), total
+
+    off, nt, topo, pc, total = table(G)
+    assert np.array_equal(off, np.cumsum(topo) - topo) and total == topo.sum()
+    for p in {0, pop // 2, pop - 1}:
+        one = table(G[p:p + 1])
+        assert one[1][0] == nt[p] and np.array_equal(one[3][:nt[p]], pc[off[p]:off[p] + nt[p]])
