@@ -668,11 +668,13 @@ int pe_grad(pe_engine* e, const float* d_genomes, int pop, const int* h_seeds, i
     // per block, warp 0 carrying all their integrator chains at once: the longest take the pipelined
     // pass (one per 8 SMs, one per 4 SMs in a batch of at most 4 flights per SM), the next nsm a block
     // each, the rest shared.  Which flights share a block changes no bit of the result.
+    // PE_GRAD_GROUP in the environment asks for them: 0 the one-flight kernel throughout, 2 shared blocks as
+    // above, 3 a block for each flight in the shared blocks' kernel.
     const char* group_env = getenv("PE_GRAD_GROUP");
     const int group_req = group_env ? atoi(group_env) : -1;
+    const bool serial = group_req == 0 || group_req == 2 || group_req == 3;
     // The reverse pass parallel in time keeps records of every flight-step.  Where those do not fit
-    // kAdjBytes, or cannot be had, the serial kernels run, as with PE_GRAD_GROUP = 0 (one flight per
-    // block) or 2 (shared blocks).  PE_GRAD_STEPS in the environment lowers kAdjSteps: longer flights
+    // kAdjBytes, or cannot be had, the serial kernels run.  PE_GRAD_STEPS in the environment lowers kAdjSteps: longer flights
     // take the one-flight kernel (gradients within ~1e-6).  Measured at 256 x 8: 4.03 ms per call with
     // the serial kernels, 3.25 ms so; at 64 x 8: 2.63 and 1.40 ms.
     const char* steps_env = getenv("PE_GRAD_STEPS");
@@ -680,7 +682,7 @@ int pe_grad(pe_engine* e, const float* d_genomes, int pop, const int* h_seeds, i
     const int rec_steps = (std::min(want_steps, max_steps) + 31) / 32 * 32;
     const size_t rec_floats = (size_t)nf * ((size_t)rec_steps * kAdjEnt + (size_t)(rec_steps / 32) * kAdjChunk);
     const int parts = (rec_steps + kAdjPart - 1) / kAdjPart;
-    if (store_forces && group_req != 0 && group_req != 2 && rec_floats * sizeof(float) <= kAdjBytes) {
+    if (store_forces && !serial && rec_floats * sizeof(float) <= kAdjBytes) {
         if (e->g_rec.ensure(rec_floats) == cudaSuccess && e->g_after.ensure((size_t)nf * 16) == cudaSuccess &&
             e->g_items.ensure(grad_time_items(nf, rec_steps)) == cudaSuccess &&
             e->g_adj.ensure((size_t)nf * parts * kAdjStride) == cudaSuccess) {
@@ -705,7 +707,7 @@ int pe_grad(pe_engine* e, const float* d_genomes, int pop, const int* h_seeds, i
         const bool small = nf <= 4 * e->nsm;
         if (store_forces && grad_long_pass(K) && (small || a.group > 1))
             a.n_long = std::min(nf, std::max(1, a.group > 1 && small ? e->nsm / 4 : e->nsm / 8));
-        a.n_single = a.group > 1 ? e->nsm : 0;
+        a.n_single = a.group > 1 ? (group_req == 3 ? nf : e->nsm) : 0;
     }
     PE_CUDA(launch_grad(a, fa, e->nsm, e->g_fwd_bps, e->wide_bps, e->g_rev_grid, s, e->ev[2]));
     PE_CUDA(record_event(e->ev[3], s));

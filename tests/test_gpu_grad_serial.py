@@ -1,0 +1,53 @@
+"""pe_grad's serial reverse kernels, which take the calls that the pass parallel in time does not: flights that
+share blocks, the pipelined pass of the longest ones, and the line between the two kinds of pass."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SEEDS = list(range(25, 33))
+
+
+def _run(torch, e, G, seeds, max_steps=3600, K=60, vary=0):
+    """Objectives, gradients and distances of a call, and how many kernels it launched."""
+    n, S = G.shape[0], len(seeds)
+    grad, obj, dist = (torch.full(s, 3.0, device="cuda") for s in ((n, 35), (n,), (n * S,)))
+    e.grad(torch.from_numpy(np.ascontiguousarray(G)).cuda(), n, seeds, grad, vary=vary, max_steps=max_steps,
+           checkpoint_every=K, d_obj=obj, d_dist=dist)
+    torch.cuda.synchronize()
+    return obj.cpu().numpy(), grad.cpu().numpy(), dist.cpu().numpy(), e.last_timing()["launches"]
+
+
+def _norms(a, b):
+    return np.linalg.norm(a.astype(np.float64) - b, axis=1) <= 1e-5 * np.linalg.norm(b.astype(np.float64), axis=1)
+
+
+@pytest.mark.parametrize("pop, nseeds, max_steps, K, vary", [(256, 8, 3600, 60, 0), (101, 3, 2400, 7, 0), (101, 3, 2400, 61, 0),
+                                                             (101, 3, 2400, 96, 0), (64, 3, 2400, 60, 1), (64, 3, 2400, 97, 0)])
+def test_shared_blocks_change_nothing(cuda, engine, oracle, monkeypatch, pop, nseeds, max_steps, K, vary):
+    """The serial kernels with the flights two to a block (PE_GRAD_GROUP=2; rebuilt a segment ahead up to
+    checkpoints every 60 steps, not so up to 96, not shared beyond) and with a block each (3) give the same
+    objectives, distances and gradients bit for bit; the one-flight kernel (0), whose sums run over four warps
+    instead of three, the same objectives and distances and gradients to 1e-5 of their norm."""
+    G = oracle.grand(4, pop)
+    usual, out = _run(cuda, engine, G, SEEDS[:nseeds], max_steps, K, vary), {}
+    for group in ("2", "3", "0"):
+        monkeypatch.setenv("PE_GRAD_GROUP", group)
+        out[group] = _run(cuda, engine, G, SEEDS[:nseeds], max_steps, K, vary)
+    for k in range(4):
+        np.testing.assert_array_equal(out["2"][k], out["3"][k])
+    for k in (0, 2):
+        np.testing.assert_array_equal(out["0"][k], out["2"][k])
+    assert _norms(out["0"][1], out["2"][1]).all()
+    assert usual[3] > out["2"][3]  # not the pass parallel in time, which has four kernels more
+
+
+def test_longest_flights_pass(cuda, engine, oracle, monkeypatch):
+    """A small batch gives its longest flights a block of three roles each, a large one fewer of them: 24 genomes
+    alone (192 flights) and among 256, objectives and distances bit for bit, gradients to 1e-5 of their norm."""
+    monkeypatch.setenv("PE_GRAD_GROUP", "2")
+    G = oracle.grand(4, 256)
+    some, all_ = _run(cuda, engine, G[100:124], SEEDS), _run(cuda, engine, G, SEEDS)
+    np.testing.assert_array_equal(some[0], all_[0][100:124])
+    np.testing.assert_array_equal(some[2], all_[2][800:992])
+    assert _norms(some[1], all_[1][100:124]).all()
