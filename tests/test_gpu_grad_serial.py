@@ -51,3 +51,20 @@ def test_longest_flights_pass(cuda, engine, oracle, monkeypatch):
     np.testing.assert_array_equal(some[0], all_[0][100:124])
     np.testing.assert_array_equal(some[2], all_[2][800:992])
     assert _norms(some[1], all_[1][100:124]).all()
+
+
+@pytest.mark.parametrize("steps", [31, 32, 33, 63, 64, 65, 95, 96, 97, 127, 128, 129, 257])
+@pytest.mark.parametrize("knob", [None, "PE_GRAD_STEPS"])
+def test_parts_and_stages(cuda, engine, oracle, monkeypatch, steps, knob):
+    """Horizons about the chunks of 32 steps, the Jacobians' items of 64, the panels' stages of 96 and parts of
+    128, and the same lengths as the limit beyond which a flight takes the serial kernel."""
+    G = oracle.grand(31, 60)
+    monkeypatch.setenv("PE_GRAD_GROUP", "2")
+    want = _run(cuda, engine, G, SEEDS[:4], 700 if knob else steps)
+    monkeypatch.delenv("PE_GRAD_GROUP")
+    if knob:
+        monkeypatch.setenv(knob, str(steps))
+    got = _run(cuda, engine, G, SEEDS[:4], 700 if knob else steps)
+    for k in (0, 2):
+        np.testing.assert_array_equal(got[k], want[k])
+    assert _norms(got[1], want[1]).all() and got[3] > want[3]
