@@ -85,9 +85,10 @@ typedef struct pe_engine pe_engine;
  *                  reference's 128-thread order (src/sim.cu:134-176).
  *   formulation 1: the same physics in the body frame, about half the operations per panel;
  *                  results agree with formulation 0 to rounding (the default).
- * In formulation 1 with lanes = 16, reg_cap = 0 or 3 and blocks = 0 the kernels of a one-launch batch are
- * chosen by its flights per SM (a block per flight, 32 lanes, four flights per warp), and a batch of at most
- * 192 flights per SM in several launches flies 32 lanes per flight: the same results, sooner.
+ * In the default shape (formulation 1, lanes 16, warps 1, reg_cap 3, blocks 0) the kernels of a one-launch batch
+ * are chosen by its flights per SM (a block per flight, 32 lanes, four flights per warp).  A batch of at most 192
+ * flights per SM is flown so whatever its warps are, and with reg_cap 0 too; in several launches it flies 32 lanes
+ * per flight.  The same results, sooner.  Any other shape flies as it is given.
  * Default: lanes 16, warps 1, chunk 7200, blocks 0, use_graph 0, formulation 1, reg_cap 3. */
 typedef struct {
     int lanes;       /* lanes per flight: 16 or 32 (formulation 0: 32 only) */

@@ -291,9 +291,15 @@ int enqueue_fly_default(pe_engine* e, int pop, int nseeds, int vary, int max_ste
     return PE_OK;
 }
 
-// Whether a configuration leaves the kernel to the engine: the default shape in one launch.
-bool default_shape(const pe_config& c, int max_steps) {
-    return c.formulation == 1 && c.lanes == 16 && (c.reg_cap == 0 || c.reg_cap == 3) && c.blocks == 0 && max_steps <= c.chunk;
+// Whether a configuration leaves the kernels of a batch of at most kOwnFlights flights per SM to the engine.
+bool uncapped16(const pe_config& c) {
+    return c.formulation == 1 && c.lanes == 16 && (c.reg_cap == 0 || c.reg_cap == 3) && c.blocks == 0;
+}
+// Above that only the default shape does: the others fly as they are given (8,192 x 8 in one launch: 10.6 ms by the
+// engine's choice, 14.4 to 14.8 by 16 lanes in blocks of one to eight warps).
+constexpr long long kOwnFlights = 192;
+bool own_choice(const pe_engine* e, const pe_config& c, long long flights) {
+    return uncapped16(c) && ((c.warps == 1 && c.reg_cap == 3) || flights <= kOwnFlights * e->nsm);
 }
 
 // Enqueue the flights of pop x nseeds (plane table already prepared on this stream).
@@ -301,12 +307,13 @@ int enqueue_fly(pe_engine* e, int pop, int nseeds, int vary, int max_steps, floa
                 cudaStream_t s, int* launches) {
     pe_config c = e->cfg;
     const int nchunks = (max_steps + c.chunk - 1) / c.chunk;
-    if (default_shape(c, max_steps))
+    const long long flights = (long long)pop * nseeds;
+    if (nchunks == 1 && own_choice(e, c, flights))
         return enqueue_fly_default(e, pop, nseeds, vary, max_steps, dist, steps, s, launches);
-    // The default shape in several launches: a batch of at most 192 flights per SM is bound by its longest
-    // flights, whose steps finish sooner at 32 lanes (1,024 x 8 in 600-step launches: 3.0 against 3.6 ms; 15-23 %
-    // below 160 flights per SM, even near 215, 16 lanes ahead from 320).
-    if (default_shape(c, c.chunk) && (long long)pop * nseeds <= 192LL * e->nsm) {
+    // In several launches a batch of at most 192 flights per SM is bound by its longest flights, whose steps
+    // finish sooner at 32 lanes (1,024 x 8 in 600-step launches: 3.0 against 3.6 ms; 15-23 % below 160 flights
+    // per SM, even near 215, 16 lanes ahead from 320).
+    if (uncapped16(c) && flights <= kOwnFlights * e->nsm) {
         c.lanes = 32;
         c.warps = 4;
         c.reg_cap = 0;

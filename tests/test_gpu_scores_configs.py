@@ -195,3 +195,20 @@ def test_c2_batched_shapes_against_oracle(cuda, pe, oracle):
     rho = spearman(a["scores"][sample], oracle.robust_scores(rd, len(sample), S))
     print("8192 x 8 sample of %d flights vs oracle: within 0.5%% %.5f, spearman %.9f" % (rd.size, within, rho))
     assert within >= 0.99 and rho >= 0.999
+
+
+@pytest.mark.parametrize("shape", [dict(warps=1), dict(warps=2), dict(warps=4), dict(warps=8)])
+def test_explicit_shapes_of_large_batches(cuda, pe, oracle, shape):
+    """Above 192 flights per SM only the default shape leaves the kernels to the engine (four flights per warp,
+    then a block per flight); 16 lanes with other warps fly as they are given, in one launch, bit for bit."""
+    torch = cuda
+    pop, seeds = 8192, [3, 4, 5, 6, 7, 8, 9, 10]
+    G, out = oracle.grand(8, pop), []
+    for kw, flights in ((dict(lanes=16, reg_cap=0, **shape), 1), ({}, 2)):
+        e = pe.Engine(0)
+        e.set_config(**kw)
+        out.append(eval_gpu(torch, e, G, seeds, max_steps=900))
+        assert e.last_timing()["launches"] == 3 + flights + 1
+        e.close()
+    for k in ("dist", "steps", "scores"):
+        assert np.array_equal(out[0][k].view(np.uint32), out[1][k].view(np.uint32)), k
