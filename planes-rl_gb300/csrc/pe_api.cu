@@ -302,6 +302,15 @@ bool own_choice(const pe_engine* e, const pe_config& c, long long flights) {
     return uncapped16(c) && ((c.warps == 1 && c.reg_cap == 3) || flights <= kOwnFlights * e->nsm);
 }
 
+// Whether a shape stands for the kernels it runs: of those that run the same ones, one does.
+bool distinct_shape(const pe_engine* e, const pe_config& c, long long flights, int max_steps) {
+    if (c.chunk < kMaxSteps && max_steps <= c.chunk) return false;  // one launch, as of 7200 steps
+    if (c.formulation == 0) return c.warps == 4;                    // what k_flight always has
+    const bool is_default = c.warps == 1 && c.reg_cap == 3;
+    if (!uncapped16(c) || flights > kOwnFlights * e->nsm) return true;
+    return is_default && max_steps <= c.chunk;  // the engine's choice; several launches fly 32 lanes x 4 warps
+}
+
 // Enqueue the flights of pop x nseeds (plane table already prepared on this stream).
 int enqueue_fly(pe_engine* e, int pop, int nseeds, int vary, int max_steps, float* dist, int* steps,
                 cudaStream_t s, int* launches) {
@@ -846,7 +855,7 @@ int pe_autotune(pe_engine* e, const float* d_genomes, int pop, const int* h_seed
                 pe_config c = keep;
                 c.lanes = lanes_opts[li]; c.warps = warps_opts[wi]; c.chunk = chunk_opts[ci];
                 c.blocks = 0; c.use_graph = 0; c.reg_cap = cap;
-                if (!valid_config(c)) continue;
+                if (!valid_config(c) || !distinct_shape(e, c, (long long)sample * nseeds, max_steps)) continue;
                 e->cfg = c;
                 if (blocks_for(e, c) <= 0) continue;
                 float ms = 0;

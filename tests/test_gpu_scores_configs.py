@@ -212,3 +212,21 @@ def test_explicit_shapes_of_large_batches(cuda, pe, oracle, shape):
         e.close()
     for k in ("dist", "steps", "scores"):
         assert np.array_equal(out[0][k].view(np.uint32), out[1][k].view(np.uint32)), k
+
+
+@pytest.mark.parametrize("max_steps", [500, 7200])
+def test_autotune_times_each_kernel_once(cuda, pe, oracle, max_steps):
+    """Shapes that run one and the same kernels are one candidate: the reference arithmetic always has four
+    warps; up to 192 flights per SM 16 lanes uncapped are the engine's own choice, which the default shape stands for."""
+    G = dev(cuda, oracle.grand(5, 256))
+    for formulation in (0, 1):
+        e = pe.Engine(0)
+        e.set_config(formulation=formulation, reg_cap=0, lanes=32 if formulation == 0 else 16)
+        for _ in range(4):  # a pick among equals would be by noise
+            c = e.autotune(G, 256, [1, 2], 0, max_steps)
+            assert c.chunk == 7200 or max_steps > 600
+            if formulation == 0:
+                assert c.warps == 4
+            elif c.lanes == 16 and c.reg_cap in (0, 3):
+                assert (c.warps, c.reg_cap, c.chunk) == (1, 3, 7200)
+        e.close()
