@@ -134,8 +134,8 @@ struct pe_engine {
     int graph_launches = 0;
     // occupancy cache
     int bps_cache[2][4][2][9] = {};
-    int lanes_grid = 0;  // grid of the 32-lane shape
-    int wide_bps = 0;    // blocks per SM of the block-per-flight kernel, once both default kernels are set up
+    int hand_bps = 0;  // blocks per SM of the 32-lane kernel that hands over
+    int wide_bps = 0;  // and of the block-per-flight kernel, once the default kernels are set up
     // gradient
     DevBuf<float> g_setup, g_ck, g_adj, g_ybar, g_dist, g_fsum;
     DevBuf<float> g_rec, g_after;
@@ -249,9 +249,7 @@ FlightArgs flight_args(pe_engine* e, int pop, int nseeds, int vary, int max_step
 
 int default_kernels(pe_engine* e) {  // occupancy queries and shared-memory opt-ins, outside any capture
     if (e->wide_bps) return PE_OK;
-    pe_config c = e->cfg;
-    c.blocks = 0; c.formulation = 1; c.reg_cap = 0; c.lanes = 32; c.warps = 4;
-    e->lanes_grid = blocks_for(e, c);
+    PE_CUDA(flight_hand_configure(&e->hand_bps));
     PE_CUDA(flight_quad_configure());
     PE_CUDA(flight_wide_configure(&e->wide_bps));
     return PE_OK;
@@ -277,7 +275,7 @@ int enqueue_fly_default(pe_engine* e, int pop, int nseeds, int vary, int max_ste
     a.active_out = e->list0.p;
     a.n_active_out = c + 2;
     if (per_sm <= kLanesFlights)
-        PE_CUDA(launch_flight_fast(a, FlightShape{32, 4, kMaxSteps, 0, 1, 0}, e->lanes_grid, s));
+        PE_CUDA(launch_flight_hand(a, e->nsm, e->hand_bps, s));
     else
         PE_CUDA(launch_flight_quad(a, e->nsm, s));
     a.landed = nullptr;

@@ -232,6 +232,23 @@ int flight_fast_blocks_per_sm(const FlightShape& sh) {
     return nb;
 }
 
+cudaError_t flight_hand_configure(int* bps) {
+    const size_t smem = 4 * paired_bytes<32>();
+    const void* fn = (const void*)&k_flight_fast<32, 0, false, false, true>;
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    int n = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, 128, smem);
+    *bps = n > 0 ? n : 1;
+    return e;
+}
+
+cudaError_t launch_flight_hand(const FlightArgs& a, int nsm, int bps, cudaStream_t s) {
+    if (a.rec || a.spread > 0.f || !a.landed) return cudaErrorInvalidValue;
+    k_flight_fast<32, 0, false, false, true><<<bps * nsm, 128, 4 * paired_bytes<32>(), s>>>(a);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_flight_fast(const FlightArgs& a, const FlightShape& sh, int grid, cudaStream_t s) {
     size_t smem = flight_fast_smem_bytes(sh);
     const void* fn = fast_fn(sh);
@@ -246,12 +263,6 @@ cudaError_t launch_flight_fast(const FlightArgs& a, const FlightShape& sh, int g
                                  (int)smem);
         if (e != cudaSuccess) return e;
         k_flight_fast<16, 0, true><<<grid, threads, smem, s>>>(a);
-    } else if (a.landed) {  // the engine's own choice for middling batches
-        if (sh.lanes != 32 || sh.cap) return cudaErrorInvalidValue;
-        e = cudaFuncSetAttribute((const void*)&k_flight_fast<32, 0, false, false, true>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        k_flight_fast<32, 0, false, false, true><<<grid, threads, smem, s>>>(a);
     } else if (sh.lanes == 16) {
         launch_lanes<16>(a, sh.cap, grid, threads, smem, s);
     } else if (sh.lanes == 32) {

@@ -120,6 +120,9 @@ constexpr long long kGradLanesFlights = 192;
 // many flights, one block per SM.  flight_quad_configure once per device before the first launch.
 cudaError_t flight_quad_configure();
 cudaError_t launch_flight_quad(const FlightArgs& a, int nsm, cudaStream_t s);
+// The 32-lane shape in 4-warp blocks that hands its last flights over (pe_flight_fast.cu).
+cudaError_t flight_hand_configure(int* bps);
+cudaError_t launch_flight_hand(const FlightArgs& a, int nsm, int bps, cudaStream_t s);
 // The body-frame flight with a block per flight (pe_flight_wide.cu): few flights, or few left.
 cudaError_t flight_wide_configure(int* bps);
 cudaError_t launch_flight_wide(const FlightArgs& a, int nsm, int bps, cudaStream_t s);
