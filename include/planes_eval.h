@@ -161,15 +161,22 @@ int pe_last_timing(pe_engine* e, float* ms, int* launches);
  * contact ends the flight, src/sim.cu:198-204); other endings keep x (horizon, |y| > 300,
  * x < -50), NaN flights score -10 and oversize meshes -100, both with zero gradient.  The
  * objective is the tail-aware score of src/sim.cu:340-357 over those distances, differentiated
- * through its active set (mean, the worst ceil(S/4), the worst).  Reverse mode runs over each
- * flight with a checkpoint every checkpoint_every steps (0 = 60) and recompute of each segment,
- * forward mode over mesh -> mass_props -> panels.  Topology genes (fin layout, deck gap) get
- * zero.  Arithmetic is FP32 with the printed inertia inverted in FP64.  The forward pass is the
- * evaluation's packed body-frame flight kernel on the gradient model's IEEE set-up of each flight
- * (print variation, scenario, release); it keeps each step's body force and torque (32 B per
- * flight-step) when all of them fit in 4 GiB, so the recompute runs the model's integrator alone;
- * PE_GRAD_STORE_FORCES=0 in the environment recomputes them from the panels instead.  Objectives
- * and distances are bit-identical either way, gradients agree to ~1e-5.
+ * through its active set (mean, the worst ceil(S/4), the worst).  Topology genes (fin layout,
+ * deck gap) get zero.  Arithmetic is FP32 with the printed inertia inverted in FP64.
+ * The forward pass is the evaluation's packed body-frame flight kernels on the gradient model's IEEE
+ * set-up of each flight (print variation, scenario, release), with a checkpoint every
+ * checkpoint_every steps (0 = 60) and each step's body force and torque (32 B per flight-step,
+ * when all of them fit in 4 GiB; PE_GRAD_STORE_FORCES=0 in the environment recomputes them).
+ * The reverse pass rebuilds the states from those, differentiates all steps of all flights at
+ * once, chains the steps' 13 x 10 matrices back over each flight, and takes the plane's adjoint back to the
+ * mesh once; its genes' tangents are forward mode over the vertices.
+ * Device memory, the engine's until it is destroyed: 64 B per checkpoint, the forces, and for the
+ * reverse pass about 700 B per flight-step of the horizon's first 3,072 steps, at most 9 GiB
+ * (PE_GRAD_BYTES in the environment lowers that).  Where the latter is more, or more than the device has
+ * left, or without the forces, serial kernels run instead, which recompute each segment between
+ * checkpoints and take about 10 KB per flight: more time, the same objectives and distances bit for bit,
+ * gradients within ~1e-6 of their norm (2e-5 on the worst-conditioned flights, where either is
+ * 1e-3 off FP64), without the forces ~1e-5.
  *   d_genomes [pop][35] (device), h_seeds [nseeds] host, nseeds <= 256, vary and env seeds as
  *   pe_eval_batch, max_steps <= 7200, 1 <= checkpoint_every <= 600.
  *   Outputs (device): d_grad [pop][35] (required), d_obj [pop] and d_dist [pop][nseeds]

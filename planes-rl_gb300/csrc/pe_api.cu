@@ -372,6 +372,21 @@ int enqueue_eval(pe_engine* e, const float* d_genomes, int pop, int nseeds, int 
     return PE_OK;
 }
 
+// Whether the device has the memory by which two buffers would grow, so that one that has not is asked once and
+// not made to fail an allocation, and the engine to give up the buffers it holds, on every call.
+bool has_room(const DevBuf<float>& x, size_t nx, const DevBuf<float>& y, size_t ny) {
+    size_t need = 0, have = 0, total = 0;
+    if (nx > x.cap) { need += nx; have += x.cap; }
+    if (ny > y.cap) { need += ny; have += y.cap; }
+    if (need == 0) return true;
+    size_t left = 0;
+    if (cudaMemGetInfo(&left, &total) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return true;
+    }
+    return need * sizeof(float) <= left + have * sizeof(float);
+}
+
 constexpr size_t kStageWords = 32 << 10;  // results that pe_evaluate_population brings back in one copy
 
 int check_seeds(const int* h_seeds, int nseeds) {
@@ -687,19 +702,23 @@ int pe_grad(pe_engine* e, const float* d_genomes, int pop, const int* h_seeds, i
     const char* group_env = getenv("PE_GRAD_GROUP");
     const int group_req = group_env ? atoi(group_env) : -1;
     const bool serial = group_req == 0 || group_req == 2 || group_req == 3;
-    // The reverse pass parallel in time keeps records of every flight-step.  Where those do not fit
-    // kAdjBytes, or cannot be had, the serial kernels run.  PE_GRAD_STEPS in the environment lowers kAdjSteps: longer flights
-    // take the one-flight kernel (gradients within ~1e-6).  Measured at 256 x 8: 4.03 ms per call with
-    // the serial kernels, 3.25 ms so; at 64 x 8: 2.63 and 1.40 ms.
+    // The reverse pass parallel in time keeps records of every flight-step.  Where they and what goes with
+    // them are more than kAdjBytes (PE_GRAD_BYTES in the environment lowers it) or than the device has left, the
+    // serial kernels run.  PE_GRAD_STEPS in the environment lowers kAdjSteps: longer flights take the
+    // one-flight kernel.  Measured at 256 x 8: 4.03 ms per call with the serial kernels, 3.06 ms so; at
+    // 64 x 8: 2.63 and 1.37 ms.
     const char* steps_env = getenv("PE_GRAD_STEPS");
     const int want_steps = steps_env ? std::max(1, std::min(kAdjSteps, atoi(steps_env))) : kAdjSteps;
     const int rec_steps = (std::min(want_steps, max_steps) + 31) / 32 * 32;
-    const size_t rec_floats = (size_t)nf * ((size_t)rec_steps * kAdjEnt + (size_t)(rec_steps / 32) * kAdjChunk);
     const int parts = (rec_steps + kAdjPart - 1) / kAdjPart;
-    if (store_forces && !serial && rec_floats * sizeof(float) <= kAdjBytes) {
-        if (e->g_rec.ensure(rec_floats) == cudaSuccess && e->g_after.ensure((size_t)nf * 16) == cudaSuccess &&
-            e->g_items.ensure(grad_time_items(nf, rec_steps)) == cudaSuccess &&
-            e->g_adj.ensure((size_t)nf * parts * kAdjStride) == cudaSuccess) {
+    const size_t n_rec = (size_t)nf * ((size_t)rec_steps * kAdjEnt + (size_t)(rec_steps / 32) * kAdjChunk);
+    const size_t n_after = (size_t)nf * 16, n_items = grad_time_items(nf, rec_steps), n_adj = (size_t)nf * parts * kAdjStride;
+    const char* bytes_env = getenv("PE_GRAD_BYTES");
+    const size_t bytes = bytes_env ? std::min<size_t>(kAdjBytes, strtoull(bytes_env, nullptr, 10)) : kAdjBytes;
+    const size_t more = n_rec + n_after + n_items + (size_t)nf * (parts - 1) * kAdjStride;  // than the serial kernels
+    if (store_forces && !serial && more * 4 <= bytes && has_room(e->g_rec, n_rec, e->g_adj, n_adj)) {
+        if (e->g_rec.ensure(n_rec) == cudaSuccess && e->g_after.ensure(n_after) == cudaSuccess &&
+            e->g_items.ensure(n_items) == cudaSuccess && e->g_adj.ensure(n_adj) == cudaSuccess) {
             a.rec = e->g_rec.p;
             a.rec_steps = rec_steps;
             a.adj_parts = parts;

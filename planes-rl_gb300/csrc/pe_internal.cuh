@@ -164,10 +164,10 @@ constexpr int kGradMaxK = 600;
 constexpr int kGradCounters = 9;
 // The reverse pass parallel in time (pe_grad_time.cu) keeps an entry per flight-step and a chunk of
 // matrices per 32 of them, for flights of at most kAdjSteps steps, and adds the plane's adjoints in parts
-// of kAdjPart steps; it is taken where the records fit kAdjBytes.
+// of kAdjPart steps; it is taken where all that, 705 bytes per flight-step at 3,072 steps, fits kAdjBytes.
 constexpr int kAdjEnt = 24, kAdjChunk = 4292;
 constexpr int kAdjSteps = 3072, kAdjPart = 128;  // 512 / 256 / 128 / 64: 1.62, 1.45, 1.40, 1.41 ms at 64 x 8, 3.32, 3.31, 3.25, 3.26 at 256 x 8
-constexpr size_t kAdjBytes = 8ull << 30;
+constexpr size_t kAdjBytes = 9ull << 30;  // 4,462 flights of 3,072 steps
 
 struct GradArgs {
     const float4* pc;

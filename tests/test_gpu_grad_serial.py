@@ -18,8 +18,8 @@ def _run(torch, e, G, seeds, max_steps=3600, K=60, vary=0):
     return obj.cpu().numpy(), grad.cpu().numpy(), dist.cpu().numpy(), e.last_timing()["launches"]
 
 
-def _norms(a, b):
-    return np.linalg.norm(a.astype(np.float64) - b, axis=1) <= 1e-5 * np.linalg.norm(b.astype(np.float64), axis=1)
+def _norms(a, b, tol=1e-5):
+    return np.linalg.norm(a.astype(np.float64) - b, axis=1) <= tol * np.linalg.norm(b.astype(np.float64), axis=1)
 
 
 @pytest.mark.parametrize("pop, nseeds, max_steps, K, vary", [(256, 8, 3600, 60, 0), (101, 3, 2400, 7, 0), (101, 3, 2400, 61, 0),
@@ -68,3 +68,38 @@ def test_parts_and_stages(cuda, engine, oracle, monkeypatch, steps, knob):
     for k in (0, 2):
         np.testing.assert_array_equal(got[k], want[k])
     assert _norms(got[1], want[1]).all() and got[3] > want[3]
+
+
+def test_records_that_do_not_fit(cuda, pe, oracle, monkeypatch):
+    """The pass parallel in time within a bound on its memory and the serial kernels beyond it, on one engine, back and
+    forth: objectives and distances bit for bit, gradients to 1e-5 of their norm.  40 x 8 flights of 513 steps take 320 x
+    (544 entries of 96 B, 17 chunks of 17,168 B, four more parts of 9,664 B, 64 B and 14 items) = 122,513,920 bytes."""
+    G, e = oracle.grand(31, 40), pe.Engine(0)
+    need = 320 * (544 * 96 + 17 * 17168 + 4 * 9664 + 64 + 14 * 4)
+    out = []
+    for bytes_ in (need, need - 1, None, 0):
+        if bytes_ is None:
+            monkeypatch.delenv("PE_GRAD_BYTES")
+        else:
+            monkeypatch.setenv("PE_GRAD_BYTES", str(bytes_))
+        out.append(_run(cuda, e, G, SEEDS, 513))
+    e.close()
+    for a, b in ((0, 2), (1, 3)):
+        for k in range(4):
+            np.testing.assert_array_equal(out[a][k], out[b][k])
+    for k in (0, 2):
+        np.testing.assert_array_equal(out[0][k], out[1][k])
+    assert out[0][3] > out[1][3] and _norms(out[0][1], out[1][1]).all()
+
+
+def test_records_at_their_largest(cuda, pe, oracle):
+    """About the bound itself: 557 planes x 8 flights of 3,072 steps take the pass parallel in time (8.99 GiB), 558
+    the serial kernels; objectives and distances bit for bit, gradients to 1e-5 of their norm for 98 % of the planes
+    (two float adjoints of one trajectory, amplified by the worst-conditioned flights) and 1e-3 for all."""
+    G, e = oracle.grand(31, 558), pe.Engine(0)
+    within, beyond = _run(cuda, e, G[:557], SEEDS, 3072), _run(cuda, e, G, SEEDS, 3072)
+    e.close()
+    assert within[3] > beyond[3]
+    np.testing.assert_array_equal(within[0], beyond[0][:557])
+    np.testing.assert_array_equal(within[2], beyond[2][:557 * 8])
+    assert _norms(within[1], beyond[1][:557]).mean() >= 0.98 and _norms(within[1], beyond[1][:557], 1e-3).all()
