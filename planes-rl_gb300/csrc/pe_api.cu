@@ -13,8 +13,9 @@
 
 #include <algorithm>
 #include <atomic>
+#include <memory>
+#include <new>
 #include <string>
-#include <vector>
 
 #include "../../include/planes_eval.h"
 #include "pe_internal.cuh"
@@ -122,7 +123,7 @@ struct pe_engine {
     DevBuf<float> g_dev, dist_dev, scores_dev;
     DevBuf<int> steps_dev;
     DevBuf<float> stage_dev;   // a small call's distances, steps and scores, one after the other
-    std::vector<float> stage;  // where they come back in one copy
+    std::unique_ptr<float[]> stage;  // where they come back in one copy
     DevBuf<float> audit_stats;  // pe_audit's 13 statistics
     // timing
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -546,12 +547,12 @@ int pe_evaluate_population(pe_engine* e, const float* h_genomes, int pop, const 
     // A copy to pageable memory waits for the stream and is staged by the driver: the results of a small call
     // come back in one instead of three (one plane x 8: 287 -> 269 us a call; pinned
     // memory 266, and 100 us on an engine's first call).  Results beyond kStageWords hide the copies.
-    const bool staged = words <= kStageWords;
+    if (words <= kStageWords && !e->stage) e->stage.reset(new (std::nothrow) float[kStageWords]);
+    const bool staged = words <= kStageWords && e->stage;
     float *dist = nullptr, *scores = nullptr;
     int* steps = nullptr;
     if (staged) {
         PE_CUDA(e->stage_dev.ensure(kStageWords));
-        e->stage.resize(kStageWords);
         dist = e->stage_dev.p;
         steps = reinterpret_cast<int*>(dist + nf);
         scores = dist + 2 * nf;
@@ -568,8 +569,8 @@ int pe_evaluate_population(pe_engine* e, const float* h_genomes, int pop, const 
     int rc = pe_eval_batch(e, e->g_dev.p, pop, h_seeds, nseeds, vary, max_steps, dist, steps, h_scores ? scores : nullptr, s);
     if (rc != PE_OK) return rc;
     if (staged) {
-        const float* got = e->stage.data();
-        PE_CUDA(cudaMemcpyAsync(e->stage.data(), dist, sizeof(float) * words, cudaMemcpyDeviceToHost, s));
+        const float* got = e->stage.get();
+        PE_CUDA(cudaMemcpyAsync(e->stage.get(), dist, sizeof(float) * words, cudaMemcpyDeviceToHost, s));
         PE_CUDA(cudaStreamSynchronize(s));
         if (h_dist) memcpy(h_dist, got, sizeof(float) * nf);
         if (h_steps) memcpy(h_steps, got + nf, sizeof(int) * nf);
