@@ -94,7 +94,8 @@ __device__ __forceinline__ void tm_store(uint32_t c32, uint32_t c8, uint32_t c2,
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
-// The loads and their wait are one statement, so no use of the words can move ahead of the wait.
+// The loads and their wait are one statement, so no use of the words can move ahead of the wait; its outputs are
+// written before its last input is read (&: none may share a register with an input).
 __device__ __forceinline__ void tm_load(uint32_t c32, uint32_t c8, uint32_t c2, TmWords& x) {
     uint32_t* w = x.w;
     asm volatile(
@@ -103,12 +104,12 @@ __device__ __forceinline__ void tm_load(uint32_t c32, uint32_t c8, uint32_t c2, 
         "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%32, %33, %34, %35, %36, %37, %38, %39}, [%43];\n\t"
         "tcgen05.ld.sync.aligned.32x32b.x2.b32 {%40, %41}, [%44];\n\t"
         "tcgen05.wait::ld.sync.aligned;"
-        : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]), "=r"(w[8]),
-          "=r"(w[9]), "=r"(w[10]), "=r"(w[11]), "=r"(w[12]), "=r"(w[13]), "=r"(w[14]), "=r"(w[15]), "=r"(w[16]),
-          "=r"(w[17]), "=r"(w[18]), "=r"(w[19]), "=r"(w[20]), "=r"(w[21]), "=r"(w[22]), "=r"(w[23]), "=r"(w[24]),
-          "=r"(w[25]), "=r"(w[26]), "=r"(w[27]), "=r"(w[28]), "=r"(w[29]), "=r"(w[30]), "=r"(w[31]), "=r"(w[32]),
-          "=r"(w[33]), "=r"(w[34]), "=r"(w[35]), "=r"(w[36]), "=r"(w[37]), "=r"(w[38]), "=r"(w[39]), "=r"(w[40]),
-          "=r"(w[41])
+        : "=&r"(w[0]), "=&r"(w[1]), "=&r"(w[2]), "=&r"(w[3]), "=&r"(w[4]), "=&r"(w[5]), "=&r"(w[6]), "=&r"(w[7]), "=&r"(w[8]),
+          "=&r"(w[9]), "=&r"(w[10]), "=&r"(w[11]), "=&r"(w[12]), "=&r"(w[13]), "=&r"(w[14]), "=&r"(w[15]), "=&r"(w[16]),
+          "=&r"(w[17]), "=&r"(w[18]), "=&r"(w[19]), "=&r"(w[20]), "=&r"(w[21]), "=&r"(w[22]), "=&r"(w[23]), "=&r"(w[24]),
+          "=&r"(w[25]), "=&r"(w[26]), "=&r"(w[27]), "=&r"(w[28]), "=&r"(w[29]), "=&r"(w[30]), "=&r"(w[31]), "=&r"(w[32]),
+          "=&r"(w[33]), "=&r"(w[34]), "=&r"(w[35]), "=&r"(w[36]), "=&r"(w[37]), "=&r"(w[38]), "=&r"(w[39]), "=&r"(w[40]),
+          "=&r"(w[41])
         : "r"(c32), "r"(c8), "r"(c2)
         : "memory");
 }
