@@ -15,7 +15,7 @@
 // a monoplane) live in its own lane of TMEM, 12 x 42 of the 512 columns, written by tcgen05.st when the
 // flight is staged and read back each step by tcgen05.ld.  The other pairs of a biplane (76 at most)
 // stay in shared memory, 4.3 KB per flight, beside the flight's state and constants, which leave the
-// registers to the panel part (136 of them, no spills).
+// registers to the panel part (142 of them, no spills).
 //
 // Bound: register reads.  A packed FMA of three register operands reads six registers through two
 // banks, three cycles instead of the pipe's two; per flight-step 172 packed and 67 scalar FMA-pipe
@@ -123,7 +123,6 @@ __device__ __forceinline__ f2 word2(const TmWords& x, int i) {
 // and the step's rates (186.3 to 184.9 ms at 100,000 x 12; loaded as packed pairs instead: 176.3 to 174.4).
 __device__ __forceinline__ unsigned uniform_(unsigned x) { return __reduce_or_sync(0xffffffffu, x); }
 __device__ __forceinline__ int uniform_(int x) { return (int)uniform_((unsigned)x); }
-__device__ __forceinline__ float uniform_(float x) { return __uint_as_float(uniform_(__float_as_uint(x))); }
 
 __device__ __forceinline__ f2 bcu(unsigned x) {
     f2 r;
@@ -172,8 +171,6 @@ __global__ void __launch_bounds__(32 * kQuadWarps, 1) k_flight_quad(FlightArgs a
     // a warp reaches the 32 TMEM lanes of its quarter; its four flights' columns follow its turn there
     const uint32_t tm = uniform_(s_tm) + ((uint32_t)(warp & 3) << 21);
     const int tm_first = (warp >> 2) * kQuadFlights;
-    const int n_work = uniform_(a.active_in ? *a.n_active_in : a.n_flights);
-    const int end = min(a.step_end, a.max_steps);
 
     WindLane wl = wind_lane(lane, 0.0f);  // of this lane's slot, as
     int flight = -1, step = 0;
@@ -187,15 +184,14 @@ __global__ void __launch_bounds__(32 * kQuadWarps, 1) k_flight_quad(FlightArgs a
             int f = 0;
             if (lane == 0) f = atomicAdd(a.work, 1);
             f = uniform_(f);
-            if (f >= n_work) { more = false; break; }
-            const int fl = a.active_in ? uniform_(a.active_in[f]) : f;
-            const int p = fl / a.nseeds, s = fl - p * a.nseeds;
+            if (f >= a.n_flights) { more = false; break; }
+            const int p = f / a.nseeds, s = f - p * a.nseeds;
             const int nt = uniform_(a.plane_nt[p]);
             if (nt <= 0) {
                 if (lane == 0) {
-                    a.dist[fl] = -100.0f;
-                    a.steps[fl] = 0;
-                    if (a.landed) atomicAdd(a.landed, 1);
+                    a.dist[f] = -100.0f;
+                    a.steps[f] = 0;
+                    atomicAdd(a.landed, 1);
                 }
                 continue;
             }
@@ -206,11 +202,8 @@ __global__ void __launch_bounds__(32 * kQuadWarps, 1) k_flight_quad(FlightArgs a
             Scenario sc;
             StateWords nst;
             fast_setup(a, p, s, &nfc.fc, &cg, &air_rho, &wp, &wr, &pmp, &sc);
-            if (a.step_begin == 0)
-                release(sc, pmp, cg, &nst.st);
-            else
-                nst.st = a.state[fl];
-            if (g == slot) { flight = fl; step = nst.st.step; wl = wind_lane(lane, nfc.fc.phase); }
+            release(sc, pmp, cg, &nst.st);
+            if (g == slot) { flight = f; step = 0; wl = wind_lane(lane, nfc.fc.phase); }
             if (lane == 0) {
 #pragma unroll
                 for (int i = 0; i < 6; i++) sf[slot].fc[i] = nfc.v[i];
@@ -387,22 +380,16 @@ __global__ void __launch_bounds__(32 * kQuadWarps, 1) k_flight_quad(FlightArgs a
                 for (int i = 0; i < 4; i++) sf[g].st[i] = sw.v[i];
             }
             __syncwarp();
-            leave = mine && (done || step >= end);
+            leave = mine && done;
             if (leave && (lane & 7) == 0) {
-                if (done) {
-                    a.dist[flight] = fit;
-                    a.steps[flight] = step;
-                    if (a.landed) atomicAdd(a.landed, 1);
-                } else if (a.active_out) {
-                    st.step = step;
-                    a.state[flight] = st;
-                    a.active_out[atomicAdd(a.n_active_out, 1)] = flight;
-                }
+                a.dist[flight] = fit;
+                a.steps[flight] = step;
+                atomicAdd(a.landed, 1);
             }
             // few flights left in the whole launch: hand this warp's over (judged on a count that was asked
             // for eight steps before, so that no step waits for it)
-            if (a.landed && !more && (++tick & 7) == 0) {
-                give = n_work - uniform_(seen) <= a.hand_over;
+            if (!more && (++tick & 7) == 0) {
+                give = a.n_flights - uniform_(seen) <= a.hand_over;
                 seen = *(volatile int*)a.landed;
             }
         } while (!give && !__any_sync(0xffffffffu, leave));
@@ -437,7 +424,10 @@ cudaError_t flight_quad_configure() {
 }
 
 cudaError_t launch_flight_quad(const FlightArgs& a, int nsm, cudaStream_t s) {
-    if (a.rec || a.spread > 0.f || a.grad_setup) return cudaErrorInvalidValue;
+    // whole flights from their release, the last ones handed over
+    if (a.rec || a.spread > 0.f || a.grad_setup || a.active_in || a.step_begin != 0 || a.step_end < a.max_steps ||
+        !a.landed || !a.active_out || !a.n_active_out)
+        return cudaErrorInvalidValue;
     k_flight_quad<<<nsm, 32 * kQuadWarps, kQuadSmem, s>>>(a);
     return cudaGetLastError();
 }

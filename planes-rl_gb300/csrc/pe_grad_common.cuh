@@ -111,42 +111,6 @@ __device__ __forceinline__ void load_fsum(const float* src, F3* F, F3* T) {
 }
 __device__ __forceinline__ void put3(float* d, F3 v) { d[0] = v.x; d[1] = v.y; d[2] = v.z; }
 __device__ __forceinline__ F3 get3(const float* d) { return pg::v3(d[0], d[1], d[2]); }
-
-// An entry of the pipelined passes (kPEnt floats): the state before a step, the step's body
-// force and torque (written by the rebuild) and its step_pre values (written one iteration later):
-//   [0..13] pos q vel w t  [16..18] Fb  [19..21] Tb  [24..26] va  [28..30] vb
-//   the gust Jacobian J (row-major) in the gaps [14] [15] [22] [23] [27] [31] [32] [33] [34]
-constexpr int kPEnt = 36;
-__device__ __forceinline__ void put_pent_post(float* e, const FSt& s, F3 F, F3 T) {
-    store_state16(e, s);
-    store_fsum(e + 16, F, T);
-}
-__device__ __forceinline__ void put_pent_pre(float* e, const pg::Pre<float>& q, const float (*J)[3]) {
-    e[14] = J[0][0]; e[15] = J[0][1]; e[22] = J[0][2];
-    e[23] = J[1][0]; e[27] = J[1][1]; e[31] = J[1][2];
-    e[32] = J[2][0]; e[33] = J[2][1]; e[34] = J[2][2];
-    put3(e + 24, q.va);
-    put3(e + 28, q.vb);
-}
-__device__ __forceinline__ void get_pent(const float* e, FSt& s, F3* F, F3* T, pg::Pre<float>& q, float (*J)[3]) {
-    const float4* e4 = reinterpret_cast<const float4*>(e);
-    const float4 a = e4[0], b = e4[1], c = e4[2], d = e4[3], f0 = e4[4], f1 = e4[5], v0 = e4[6], v1 = e4[7],
-                 j2 = e4[8];
-    s.pos = pg::v3(a.x, a.y, a.z);
-    s.q[0] = a.w; s.q[1] = b.x; s.q[2] = b.y; s.q[3] = b.z;
-    s.vel = pg::v3(b.w, c.x, c.y);
-    s.w = pg::v3(c.z, c.w, d.x);
-    s.t = d.y;
-    J[0][0] = d.z; J[0][1] = d.w;
-    *F = pg::v3(f0.x, f0.y, f0.z);
-    *T = pg::v3(f0.w, f1.x, f1.y);
-    J[0][2] = f1.z; J[1][0] = f1.w;
-    q.va = pg::v3(v0.x, v0.y, v0.z);
-    J[1][1] = v0.w;
-    q.vb = pg::v3(v1.x, v1.y, v1.z);
-    J[1][2] = v1.w;
-    J[2][0] = j2.x; J[2][1] = j2.y; J[2][2] = j2.z;
-}
 }  // namespace
 
 }  // namespace pe

@@ -56,7 +56,7 @@ __device__ __forceinline__ void load_ent(const float* e, FSt& s, F3* F, F3* T, F
     s = load_state16(e);
     *F = pg::v3(f0.x, f0.y, f0.z);
     *T = pg::v3(f0.w, f1.x, f1.y);
-    *vb = pg::v3(d.w, f1.z, f1.w);
+    if (vb) *vb = pg::v3(d.w, f1.z, f1.w);
 }
 // Whether this pass differentiates flight f (the serial kernel takes the longer ones).
 __device__ __forceinline__ bool adj_takes(const GradArgs& a, int f) {
@@ -276,8 +276,8 @@ __global__ void __launch_bounds__(kJacSteps, kJacBlocks) k_adj_jacobian(GradArgs
         // position's own adjoint passes through and is the chain's to add.
         const pg::FlightP<float> P = setup_flightp(a, f);
         FSt st;
-        F3 Fb, Tb, vb_;
-        load_ent(e, st, &Fb, &Tb, &vb_);
+        F3 Fb, Tb;
+        load_ent(e, st, &Fb, &Tb, nullptr);
         pg::Pre<float> pr;
         float Jw[3][3];
         pg::step_pre(P, st, pr, Jw);
@@ -388,7 +388,7 @@ struct PanAcc {
 };
 
 // The adjoints of a pair's panels at one step, added to acc.
-__device__ __forceinline__ void pan_pair(const PanPair& p, const f2* k, float cfs, f2 cf, PanAcc& acc) {
+__device__ __forceinline__ void pan_pair(const PanPair& p, const f2* k, f2 cf, PanAcc& acc) {
     const f2 vx = fma2(k[4], p.rz, fma2(k[8], p.ry, k[0]));
     const f2 vy = fma2(k[5], p.rx, fma2(k[6], p.rz, k[1]));
     const f2 vz = fma2(k[3], p.ry, fma2(k[7], p.rx, k[2]));
@@ -470,8 +470,8 @@ __global__ void __launch_bounds__(kPanThreads, 5) k_adj_panels(GradArgs a, long 
     const int p = f / a.nseeds, nt = a.plane_nt[p], off = a.plane_off[p], n = min(a.steps[f], first + kAdjPart);
     const float* rec = a.setup + (size_t)f * kGradSetupFloats;
     const F3 cg = pg::v3(rec[22], rec[23], rec[24]);
-    const float rho = rec[25], wp = rec[26], wr = rec[27], cfs = rec[17];
-    const f2 cf = bc(cfs);
+    const float rho = rec[25], wp = rec[26], wr = rec[27];
+    const f2 cf = bc(rec[17]);
     PanPair pp[2];
     PanAcc acc[2];
 #pragma unroll
@@ -548,7 +548,7 @@ __global__ void __launch_bounds__(kPanThreads, 5) k_adj_panels(GradArgs a, long 
                     k[2 * q + 1] = x.y;
                 }
 #pragma unroll
-                for (int c = 0; c < NC; c++) pan_pair(pp[c], k, cfs, cf, acc[c]);
+                for (int c = 0; c < NC; c++) pan_pair(pp[c], k, cf, acc[c]);
             }
         }
     };
