@@ -705,9 +705,17 @@ int pe_grad(pe_engine* e, const float* d_genomes, int pop, const int* h_seeds, i
     const bool serial = group_req == 0 || group_req == 2 || group_req == 3;
     // The reverse pass parallel in time keeps records of every flight-step.  Where they and what goes with
     // them are more than kAdjBytes (PE_GRAD_BYTES in the environment lowers it) or than the device has left, the
-    // serial kernels run.  PE_GRAD_STEPS in the environment lowers kAdjSteps: longer flights take the
-    // one-flight kernel.  Measured at 256 x 8: 4.03 ms per call with the serial kernels, 3.06 ms so; at
-    // 64 x 8: 2.63 and 1.37 ms.
+    // serial kernels run.  PE_GRAD_STEPS in the environment lowers kAdjSteps (longer flights take the
+    // one-flight kernel) and takes the pass at any horizon.  Measured at 256 x 8: 4.03 ms per call with the
+    // serial kernels, 3.06 ms so; at 64 x 8: 2.63 and 1.37 ms.
+    // A short horizon does not pay for its four more launches and its items of 64 steps.  Milliseconds of the
+    // serial kernels / parallel in time by steps:
+    //   flights     16            33            48            64            65            80            96
+    //        64   0.18 / 0.30   0.23 / 0.32   0.27 / 0.33   0.34 / 0.36   0.33 / 0.38   0.37 / 0.39   0.43 / 0.39
+    //       512   0.24 / 0.35   0.32 / 0.39   0.40 / 0.42   0.49 / 0.45   0.51 / 0.46   0.51 / 0.44   0.60 / 0.47
+    //     2,048   0.40 / 0.50   0.55 / 0.59   0.69 / 0.64   0.83 / 0.69   0.83 / 0.83   0.96 / 0.89   1.08 / 0.94
+    //     8,000   1.10 / 1.46   1.54 / 1.67   1.89 / 1.85   2.33 / 2.04   2.35 / 2.58   2.70 / 2.76   3.03 / 2.94
+    const bool pays = max_steps >= 96 || (max_steps > 48 && nf > 2 * e->nsm && (max_steps <= 64 || nf <= 16 * e->nsm));
     const char* steps_env = getenv("PE_GRAD_STEPS");
     const int want_steps = steps_env ? std::max(1, std::min(kAdjSteps, atoi(steps_env))) : kAdjSteps;
     const int rec_steps = (std::min(want_steps, max_steps) + 31) / 32 * 32;
@@ -717,7 +725,7 @@ int pe_grad(pe_engine* e, const float* d_genomes, int pop, const int* h_seeds, i
     const char* bytes_env = getenv("PE_GRAD_BYTES");
     const size_t bytes = bytes_env ? std::min<size_t>(kAdjBytes, strtoull(bytes_env, nullptr, 10)) : kAdjBytes;
     const size_t more = n_rec + n_after + n_items + (size_t)nf * (parts - 1) * kAdjStride;  // than the serial kernels
-    if (store_forces && !serial && more * 4 <= bytes && has_room(e->g_rec, n_rec, e->g_adj, n_adj)) {
+    if (store_forces && !serial && (pays || steps_env) && more * 4 <= bytes && has_room(e->g_rec, n_rec, e->g_adj, n_adj)) {
         if (e->g_rec.ensure(n_rec) == cudaSuccess && e->g_after.ensure(n_after) == cudaSuccess &&
             e->g_items.ensure(n_items) == cudaSuccess && e->g_adj.ensure(n_adj) == cudaSuccess) {
             a.rec = e->g_rec.p;

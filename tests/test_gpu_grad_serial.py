@@ -62,8 +62,7 @@ def test_parts_and_stages(cuda, engine, oracle, monkeypatch, steps, knob):
     monkeypatch.setenv("PE_GRAD_GROUP", "2")
     want = _run(cuda, engine, G, SEEDS[:4], 700 if knob else steps)
     monkeypatch.delenv("PE_GRAD_GROUP")
-    if knob:
-        monkeypatch.setenv(knob, str(steps))
+    monkeypatch.setenv("PE_GRAD_STEPS", str(steps if knob else 3072))  # set, it takes the pass at any horizon
     got = _run(cuda, engine, G, SEEDS[:4], 700 if knob else steps)
     for k in (0, 2):
         np.testing.assert_array_equal(got[k], want[k])
@@ -103,3 +102,20 @@ def test_records_at_their_largest(cuda, pe, oracle):
     np.testing.assert_array_equal(within[0], beyond[0][:557])
     np.testing.assert_array_equal(within[2], beyond[2][:557 * 8])
     assert _norms(within[1], beyond[1][:557]).mean() >= 0.98 and _norms(within[1], beyond[1][:557], 1e-3).all()
+
+
+@pytest.mark.parametrize("pop, nseeds, short, longer", [(8, 8, (1, 48, 64, 65, 95), (96,)), (64, 8, (1, 48), (49, 64, 65, 95, 96)),
+                                                        (400, 8, (1, 48, 65, 95), (49, 64, 96))])
+def test_short_horizons_take_the_serial_kernels(cuda, engine, oracle, monkeypatch, pop, nseeds, short, longer):
+    """Where the pass parallel in time does not pay for its launches and its items of 64 steps: below 96 steps for few
+    flights, below 49 for all, from 65 to 95 for more than 16 per SM."""
+    G = oracle.grand(31, pop)
+    for steps in short + longer:
+        monkeypatch.delenv("PE_GRAD_GROUP", raising=False)
+        got = _run(cuda, engine, G, SEEDS[:nseeds], steps)
+        monkeypatch.setenv("PE_GRAD_GROUP", "2")
+        want = _run(cuda, engine, G, SEEDS[:nseeds], steps)
+        for k in (0, 2):
+            np.testing.assert_array_equal(got[k], want[k])
+        assert _norms(got[1], want[1]).all()
+        assert (got[3] > want[3]) == (steps in longer), steps
