@@ -204,3 +204,25 @@ def test_panel_offsets(cuda, pe, oracle, pop):
     for p in {0, pop // 2, pop - 1}:
         one = table(G[p:p + 1])
         assert one[1][0] == nt[p] and np.array_equal(one[3][:nt[p]], pc[off[p]:off[p] + nt[p]])
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("pop, nseeds", [(1, 1), (1, 8), (40, 8), (80, 8), (310, 8)])  # one to four flights per block
+def test_objective_few_flights(cuda, pe, oracle, precision, pop, nseeds):
+    """pe_objective's flights do not depend on how many share a block: the first planes as they fly alone."""
+    torch = cuda
+    G, seeds = oracle.grand(53, pop), list(range(2, 2 + nseeds))
+    e = pe.Engine(0)
+
+    def dist(g):
+        n = g.shape[0]
+        obj, d = (torch.empty(k, dtype=torch.float64, device="cuda") for k in (n, nseeds * n))
+        e.objective(torch.from_numpy(np.ascontiguousarray(g)).cuda(), n, seeds, precision=precision, max_steps=700, d_obj=obj, d_dist=d)
+        torch.cuda.synchronize()
+        return obj.cpu().numpy(), d.cpu().numpy()
+
+    obj, d = dist(G)
+    for p in range(min(pop, 4)):
+        alone = dist(G[p:p + 1])
+        assert np.array_equal(alone[0], obj[p:p + 1]) and np.array_equal(alone[1], d[p * nseeds:(p + 1) * nseeds])
+    e.close()
