@@ -94,7 +94,7 @@ typedef struct {
     int lanes;       /* lanes per flight: 16 or 32 (formulation 0: 32 only) */
     int warps;       /* warps per block of the flight kernel: 1..8 (formulation 0: always 4) */
     int chunk;       /* steps per flight launch: 1..7200 */
-    int blocks;      /* flight grid size; 0 = fill the GPU (persistent) */
+    int blocks;      /* flight grid size; 0 = fill the GPU (persistent); formulation 0 with warps > 4: warps / 4 times it */
     int use_graph;   /* 1 = replay the whole evaluation from a captured CUDA graph */
     int formulation; /* 0 = reference arithmetic, 1 = body frame */
     int reg_cap;     /* body frame only: registers capped so more flights reside per SM, 1 = 96,

@@ -6,6 +6,7 @@
 // The flights are the engine's own choice of one or two kernels (enqueue_fly_default), or in an explicit
 // shape ceil(max_steps / chunk) launches (persistent grid; each reads the previous launch's list of airborne
 // flights).  With use_graph the whole sequence is captured once per shape and replayed.
+#include <limits.h>
 #include <stdarg.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -204,7 +205,8 @@ int engine_reserve(pe_engine* e, int pop, int nflights) {
 }
 
 int blocks_for(pe_engine* e, const pe_config& c) {
-    if (c.blocks > 0) return c.blocks;
+    // a block of the reference arithmetic flies four flights, whatever its warps: a grid given with eight is for twice as many
+    if (c.blocks > 0) return c.formulation ? c.blocks : (int)std::min<long long>(INT_MAX, std::max<long long>(c.blocks, (long long)c.blocks * c.warps / 4));
     int& bps = e->bps_cache[c.formulation][c.reg_cap][c.lanes == 16 ? 0 : 1][c.warps];
     if (bps == 0) {
         FlightShape sh{c.lanes, c.warps, c.chunk, 0, c.formulation, c.reg_cap};

@@ -226,3 +226,12 @@ def test_objective_few_flights(cuda, pe, oracle, precision, pop, nseeds):
         alone = dist(G[p:p + 1])
         assert np.array_equal(alone[0], obj[p:p + 1]) and np.array_equal(alone[1], d[p * nseeds:(p + 1) * nseeds])
     e.close()
+
+
+@pytest.mark.parametrize("blocks, warps", [(1, 8), (1, 1), (5, 7), (300, 2), (1000, 8)])
+def test_reference_order_given_grid(cuda, pe, oracle, blocks, warps):
+    """The reference arithmetic in a grid that is given: as in its own, bit for bit."""
+    G, shape = oracle.grand(17, 50), dict(formulation=0, lanes=32, reg_cap=0)
+    want = _flights(cuda, pe, G, [3, 4, 5, 6], shape=shape, max_steps=700)
+    got = _flights(cuda, pe, G, [3, 4, 5, 6], shape=dict(blocks=blocks, warps=warps, **shape), max_steps=700)
+    assert all(np.array_equal(a, b) for a, b in zip(got, want))
