@@ -709,7 +709,7 @@ int pe_grad(pe_engine* e, const float* d_genomes, int pop, const int* h_seeds, i
     // them are more than kAdjBytes (PE_GRAD_BYTES in the environment lowers it) or than the device has left, the
     // serial kernels run.  PE_GRAD_STEPS in the environment lowers kAdjSteps (longer flights take the
     // one-flight kernel) and takes the pass at any horizon.  Measured at 256 x 8: 4.03 ms per call with the
-    // serial kernels, 3.06 ms so; at 64 x 8: 2.63 and 1.37 ms.
+    // serial kernels, 3.06 ms so; at 64 x 8: 2.63 and 1.30 ms.
     // A short horizon does not pay for its four more launches and its items of 64 steps.  Milliseconds of the
     // serial kernels / parallel in time by steps:
     //   flights     16            33            48            64            65            80            96

@@ -18,15 +18,17 @@
 //   (Lvb; Lw) = -G (LF; LT),  G = sum of (alpha N + beta V) N^T + gamma V V^T + nv B B^T
 // over the panels, N = B n, V = B v.
 //
-// The records take 633 bytes per flight-step (kAdjStepFloats) for the first kAdjSteps steps of every
-// flight; longer flights take the serial kernel, and so do all where the records do not fit kAdjBytes.
+// The records take 633 bytes per flight-step (kAdjEnt floats, and kAdjChunk per 32 steps) for the first
+// kAdjSteps steps of every flight; longer flights take the serial kernel, and so do all where the records and
+// the adjoints' parts do not fit kAdjBytes, and most calls of horizons below 96 steps (pe_grad).
 // Built without fast math, as pe_grad.cu.
 //
 // Measured (GB300, 256 x 8 x 3600 / 64 x 8 x 7200): states 0.05 / 0.04 ms, Jacobians 0.94 / 0.29, chain
 // 0.10 / 0.08 (with the model's adjoint in the chain, eight lanes a flight: 0.74 / 0.66), panels 0.77 /
-// 0.27 (512 steps a block: 0.81 / 0.46, for want of blocks); the call 4.03 -> 3.25 ms and 2.63 -> 1.40 ms.  The Jacobians and the panels are bound by register
-// reads (a scalar FMA of three registers takes two cycles of the two banks, a packed one three), not by
-// the pipe: 163 instructions per panel and 32 steps take 224 cycles.
+// 0.27 (512 steps a block: 0.81 / 0.46, for want of blocks); the call 4.03 -> 3.25 ms and 2.63 -> 1.40 ms, and 3.06 and 1.30 since parts of 128 steps and
+// k_grad_genome's corner adjoints.  The Jacobians and the panels are bound by register reads (a scalar FMA of
+// three registers takes two cycles of the two banks, a packed one three), not by the pipe: 163 instructions
+// per panel and 32 steps take 224 cycles.
 #include <cuda_runtime.h>
 
 #include <type_traits>
